@@ -28,6 +28,17 @@ __device__ __forceinline__ uint32_t find_job(const WaveJob* jobs, uint32_t lo, u
     return lo;
 }
 
+// A render's primary rays and paths, known beforehand: added by the thread of its first item.
+__device__ __forceinline__ void count_render(const WaveJob& J, uint32_t item)
+{
+    if (item == J.item_base) {
+        const FrameParams& P = J.P;
+        const unsigned long long n = (unsigned long long)P.w * P.h * P.batch;
+        atomicAdd(P.stats + 0, n);
+        atomicAdd(P.stats + 1, n * P.light_samples);
+    }
+}
+
 __global__ void k_batch_start(BatchCtl* ctl, cudaGraphConditionalHandle outer)
 {
     ctl->wave = 0;
@@ -72,12 +83,8 @@ __global__ void __launch_bounds__(256) k_batch_primary(BatchDev B)
             slot = J.slot_base + (g - J.item_base);
             push = primary_ray<WIDTH, MASK>(P, S, it, slot, tc);
         }
-        push_primary(S, push, slot);
-        const uint32_t mv = __ballot_sync(0xffffffffu, it.valid);
-        if (lane_id() == 0 && mv) {
-            atomicAdd(P.stats + 0, (unsigned long long)__popc(mv));
-            atomicAdd(P.stats + 1, (unsigned long long)__popc(mv) * P.light_samples);
-        }
+        push_queue(S, 1, push, slot);
+        count_render(J, g);
     }
     flush_counts(tc, &B.ctl->box_tests);
 }
@@ -180,11 +187,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_batch_primary_shade
             push = primary_shade<WIDTH, MASK>(P, S, it, slot, tc);
         }
         push_queue(S, 0, push, slot);
-        const uint32_t mv = __ballot_sync(0xffffffffu, it.valid);
-        if (lane_id() == 0 && mv) {
-            atomicAdd(P.stats + 0, (unsigned long long)__popc(mv));
-            atomicAdd(P.stats + 1, (unsigned long long)__popc(mv) * P.light_samples);
-        }
+        count_render(J, g);
     }
     flush_counts(tc, &B.ctl->box_tests);
 }

@@ -347,6 +347,78 @@ __device__ __forceinline__ bool bounce(const FrameParams& P, const PathState& S,
     return shade_run(P, S, L);
 }
 
+// The queue lengths and the counters are single words, and the atomics on one address are served
+// one after another (about 2.3 per ns over the whole GPU, measured), so a kernel of millions of
+// short warps that each add to a few of them is bound by that rate: with five atomics per warp the
+// camera pass of the 1M-sphere 1080p frame took 36 ms, with three per block of 8 warps 26 ms
+// (frame 75.0 -> 64.8 ms).  push_block and flush_block share them over a block.
+constexpr uint32_t PATH_BLOCK = 256;  // threads per block of every kernel using them
+
+// Append the slots of the block's threads with push set to queue q, in thread order, with one
+// atomic, and add the block's traversal counts to counters[0] (box tests) and counters[1]
+// (primitive tests).  Every thread of the block calls it (once per kernel).
+__device__ __forceinline__ void push_block(const PathState& S, int q, bool push, uint32_t slot,
+                                           const TraceCount& tc, unsigned long long* counters)
+{
+    constexpr uint32_t W = PATH_BLOCK / 32;
+    __shared__ uint32_t at[W], box[W], prim[W];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t m = __ballot_sync(0xffffffffu, push);
+    const uint32_t b = __reduce_add_sync(0xffffffffu, tc.box);
+    const uint32_t p = __reduce_add_sync(0xffffffffu, tc.prim);
+    if (lane == 0) {
+        at[warp] = uint32_t(__popc(m));
+        box[warp] = b;
+        prim[warp] = p;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        unsigned long long nb = 0, np = 0;
+        for (uint32_t k = 0; k < W; ++k) {
+            n += at[k];
+            nb += box[k];
+            np += prim[k];
+        }
+        if (nb | np) {
+            atomicAdd(counters, nb);
+            atomicAdd(counters + 1, np);
+        }
+        if (n) {
+            uint32_t base = atomicAdd(S.ctr + q, n);
+            for (uint32_t k = 0; k < W; ++k) {
+                const uint32_t here = at[k];
+                at[k] = base;
+                base += here;
+            }
+        }
+    }
+    __syncthreads();
+    if (push)
+        st_cs(S.queue[q] + (at[warp] + __popc(m & ((1u << lane) - 1u))), slot);
+}
+
+// Add the block's traversal counts to the counters alone (any block shape).
+__device__ __forceinline__ void flush_block(const TraceCount& tc, unsigned long long* counters)
+{
+    __shared__ unsigned long long sum[2];
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if (first)
+        sum[0] = sum[1] = 0;
+    __syncthreads();
+    const uint32_t b = __reduce_add_sync(0xffffffffu, tc.box);
+    const uint32_t p = __reduce_add_sync(0xffffffffu, tc.prim);
+    if (lane_id() == 0) {
+        atomicAdd(&sum[0], (unsigned long long)b);
+        atomicAdd(&sum[1], (unsigned long long)p);
+    }
+    __syncthreads();
+    if (first && (sum[0] | sum[1])) {
+        atomicAdd(counters, sum[0]);
+        atomicAdd(counters + 1, sum[1]);
+    }
+}
+
 // Append the lanes with push set to queue q (one atomic per warp).
 __device__ __forceinline__ void push_queue(const PathState& S, int q, bool push, uint32_t slot)
 {
@@ -359,21 +431,6 @@ __device__ __forceinline__ void push_queue(const PathState& S, int q, bool push,
         at = __shfl_sync(0xffffffffu, at, 0);
         if (push)
             st_cs(S.queue[q] + (at + __popc(m & ((1u << lane) - 1u))), slot);
-    }
-}
-
-// Append the lanes with push set to queue 1 (one atomic per warp).
-__device__ __forceinline__ void push_primary(const PathState& S, bool push, uint32_t slot)
-{
-    const uint32_t lane = lane_id();
-    const uint32_t m = __ballot_sync(0xffffffffu, push);
-    if (m) {
-        uint32_t at = 0;
-        if (lane == 0)
-            at = atomicAdd(S.ctr + 1, uint32_t(__popc(m)));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (push)
-            st_cs(S.queue[1] + (at + __popc(m & ((1u << lane) - 1u))), slot);
     }
 }
 

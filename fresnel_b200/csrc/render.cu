@@ -25,6 +25,16 @@ namespace fr {
 
 namespace {
 
+// The primary pass's rays and paths, known before it runs: added by its first thread.
+__device__ __forceinline__ void count_primary(const FrameParams& P, uint32_t thread)
+{
+    if (thread == 0u) {
+        const unsigned long long n = (unsigned long long)P.w * P.h * P.batch;
+        atomicAdd(P.stats + 0, n);
+        atomicAdd(P.stats + 1, n * P.light_samples);
+    }
+}
+
 // Primary rays of every slot of the batch, one thread per work item (primary_item order).
 template <int WIDTH, uint32_t MASK, bool PACKET = false>
 __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S)
@@ -56,13 +66,8 @@ __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S
         slot = g;
         push = primary_ray<WIDTH, MASK>(P, S, it, slot, tc);
     }
-    flush_counts(tc, P.stats + 3);
-    push_primary(S, push, slot);
-    const uint32_t mv = __ballot_sync(0xffffffffu, it.valid);
-    if (lane_id() == 0 && mv) {
-        atomicAdd(P.stats + 0, (unsigned long long)__popc(mv));
-        atomicAdd(P.stats + 1, (unsigned long long)__popc(mv) * P.light_samples);
-    }
+    push_block(S, 1, push, slot, tc, P.stats + 3);
+    count_primary(P, g);
 }
 
 // Primary rays with their first shading (device option "fuse_shade"): one thread per work item
@@ -82,13 +87,8 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(
     TraceCount tc;
     if (it.valid)
         push = primary_shade<WIDTH, MASK>(P, S, it, g, tc);
-    flush_counts(tc, P.stats + 3);
-    push_queue(S, 0, push, g);
-    const uint32_t mv = __ballot_sync(0xffffffffu, it.valid);
-    if (lane_id() == 0 && mv) {
-        atomicAdd(P.stats + 0, (unsigned long long)__popc(mv));
-        atomicAdd(P.stats + 1, (unsigned long long)__popc(mv) * P.light_samples);
-    }
+    push_block(S, 0, push, g, tc, P.stats + 3);
+    count_primary(P, g);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -411,9 +411,9 @@ __global__ void __launch_bounds__(256) k_path_extend(FrameParams P, PathState S,
                 st_cs(S.hit + (p), make_uint2(h.geom, h.prim));
             }
         }
-        if (lane == 0)
-            atomicAdd(P.stats + 0, (unsigned long long)min(CHUNK, count - base));
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(P.stats + 0, (unsigned long long)count);
     flush_counts(tc, P.stats + 3);
 }
 
@@ -428,6 +428,8 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_bounce(FramePa
     const uint32_t* queue = S.queue[q];
     const uint32_t lane = threadIdx.x & 31u;
     TraceCount tc;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(P.stats + 0, (unsigned long long)count);
     while (true) {
         uint32_t base = 0;
         if (lane == 0)
@@ -443,8 +445,6 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_bounce(FramePa
             push = bounce<WIDTH, MASK>(P, S, p, p, tc);
         }
         push_queue(S, q ^ 1, push, p);
-        if (lane == 0)
-            atomicAdd(P.stats + 0, (unsigned long long)min(32u, count - base));
     }
     flush_counts(tc, P.stats + 3);
 }
@@ -713,6 +713,16 @@ __device__ __forceinline__ C3 preview_shade(const FrameParams& P, const GeomDev&
     return c;
 }
 
+// The frame's rays (one path each), added by the launch's first thread.
+__device__ __forceinline__ void count_preview(const FrameParams& P, uint32_t ns)
+{
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+        const unsigned long long n = (unsigned long long)P.w * P.h * ns;
+        atomicAdd(P.stats + 0, n);
+        atomicAdd(P.stats + 1, n);
+    }
+}
+
 template <int WIDTH, uint32_t MASK>
 __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, uint2* hits)
 {
@@ -747,12 +757,8 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
         float q = 1.0f / float(ns);
         write_pixel(P, p, avg[0] * q, avg[1] * q, avg[2] * q, avg[3] * q);
     }
-    flush_counts(tc, P.stats + 3);
-    uint32_t m = __ballot_sync(0xffffffffu, valid);
-    if ((threadIdx.x + threadIdx.y * blockDim.x) % 32 == 0 && m) {
-        atomicAdd(P.stats + 0, (unsigned long long)__popc(m) * ns);
-        atomicAdd(P.stats + 1, (unsigned long long)__popc(m) * ns);
-    }
+    flush_block(tc, P.stats + 3);
+    count_preview(P, ns);
 }
 
 // Preview with a group of G lanes per pixel (G = 32 or 16 dividing the samples per pixel: 4x4
@@ -803,11 +809,8 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
             write_pixel(P, p, avg[0] * q, avg[1] * q, avg[2] * q, avg[3] * q);
         }
     }
-    flush_counts(tc, P.stats + 3);
-    if (valid && gl == 0u) {
-        atomicAdd(P.stats + 0, (unsigned long long)ns);
-        atomicAdd(P.stats + 1, (unsigned long long)ns);
-    }
+    flush_block(tc, P.stats + 3);
+    count_preview(P, ns);
 }
 
 // Diagnostic: trace rays[i] = (o, d) with both 4-wide traversal forms (one ray per thread, and
