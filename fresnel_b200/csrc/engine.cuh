@@ -63,6 +63,7 @@ struct GeomDev {
     float bound_radius;     // polyhedron, polygon: bounding radius about the position; mesh: the
                             // largest vertex distance from the instance origin
     const float4* face_box;  // mesh: per face its padded box in the instance frame (lo, hi)
+    uint32_t bounded;        // 1: the surface (unit orientation) lies within bound_radius
     float color_by_face;
     float outline_width;
     Mat material;
@@ -83,6 +84,8 @@ struct GridDev {
     float hx, hy, hz;     // cell size
     float ihx, ihy, ihz;  // 1 / cell size
     uint32_t geom;        // scene index of the sphere geometry
+    uint32_t n_valid;     // primitives with a finite, non-empty box
+    float mean_radius;    // root of their mean cross-section / pi
     const uint32_t* cell_start;
     const float4* ref_sphere;
     const uint32_t* ref_prim;

@@ -462,6 +462,8 @@ cudaError_t build_cells(const Src& src, uint32_t n, const Reasons& why, const Gr
         rep.reason = why.clustered;
         return cudaSuccess;
     }
+    out.mean_radius = float(std::sqrt(mean_r2));
+    out.n_valid = rep.n_valid;
     for (int k = 0; k < 3; ++k) {
         out.dims[k] = dims[k];
         out.lo[k] = flo[k];

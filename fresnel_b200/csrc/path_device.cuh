@@ -3,7 +3,7 @@
 #ifndef FR_PATH_DEVICE_CUH
 #define FR_PATH_DEVICE_CUH
 
-#include "render.hpp"
+#include "beam.cuh"
 
 namespace fr {
 namespace {
@@ -279,13 +279,26 @@ __device__ __forceinline__ bool primary_ray(const FrameParams& P, const PathStat
 // miss finishes its pixel sample as in primary_finish; a hit is shaded from registers, without
 // storing the primary ray (unless a later light sample restarts from it) or reading anything
 // back.  Returns true when the path continues (its extension ray is stored; queue it).
-template <int WIDTH, uint32_t MASK>
+// LISTS: the frame has pixel lists (beam.cuh).
+template <int WIDTH, uint32_t MASK, bool LISTS = false>
 __device__ __forceinline__ bool primary_shade(const FrameParams& P, const PathState& S,
                                               const PrimaryItem& it, uint32_t slot, TraceCount& tc)
 {
     V3 o, d;
-    camera_ray(P.cam, it.i, it.j, P.n_samples + it.k, o, d);
-    Hit h = trace_closest<WIDTH, MASK>(P.scene, o, d, PATH_TNEAR, tc);
+    Hit h;
+    if constexpr (LISTS) {
+        const uint2* list = pixel_list(P, it.i, it.j);
+        h.geom = MISS;
+        h.prim = 0;
+        if (!list_empty(list)) {
+            camera_ray(P.cam, it.i, it.j, P.n_samples + it.k, o, d);
+            if (!list_hit<MASK>(P, list, o, d, PATH_TNEAR, tc, h))
+                h = trace_closest<WIDTH, MASK>(P.scene, o, d, PATH_TNEAR, tc);
+        }
+    } else {
+        camera_ray(P.cam, it.i, it.j, P.n_samples + it.k, o, d);
+        h = trace_closest<WIDTH, MASK>(P.scene, o, d, PATH_TNEAR, tc);
+    }
     const uint2 ph = make_uint2(h.geom, h.prim);
     st_cs(S.prim_hit + (slot), ph);
     if (h.geom == MISS) {

@@ -73,8 +73,9 @@ __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S
 // Primary rays with their first shading (device option "fuse_shade"): one thread per work item
 // as k_path_primary; continuing paths go straight to the extension queue (queue 0), so the
 // frame's first shade pass is not launched.  Limited to fused_blocks<MASK> blocks of 256 threads
-// per SM.
-template <int WIDTH, uint32_t MASK>
+// per SM.  LISTS: the frame has pixel lists (a kernel of its own, so that frames without them
+// carry none of their code: path images of polygons 3% faster).
+template <int WIDTH, uint32_t MASK, bool LISTS = false>
 __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(FrameParams P, PathState S)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(
     bool push = false;
     TraceCount tc;
     if (it.valid)
-        push = primary_shade<WIDTH, MASK>(P, S, it, g, tc);
+        push = primary_shade<WIDTH, MASK, LISTS>(P, S, it, g, tc);
     push_block(S, 0, push, g, tc, P.stats + 3);
     count_primary(P, g);
 }
@@ -767,7 +768,7 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
 // nodes, where k_preview's warp holds 32 pixels whose sample loops run side by side.  Each round
 // of G samples is summed in sample order (every lane reads its group's G colours by shuffles), so
 // the pixel is the same float sum as k_preview's; the hit ids go to the same places.
-template <int WIDTH, uint32_t MASK, uint32_t G>
+template <int WIDTH, uint32_t MASK, uint32_t G, bool LISTS = false>
 __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa_n, uint2* hits)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -780,12 +781,23 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
     TraceCount tc;
     if (valid) {
         const uint32_t j = p / P.w, i = p - j * P.w;
+        const uint2* list = LISTS ? pixel_list(P, i, j) : nullptr;
+        const bool empty = LISTS && list_empty(list);
         float avg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (uint32_t base = 0; base < ns; base += G) {
             const uint32_t sample = base + gl;
             V3 o, d;
-            camera_ray(P.cam, i, j, sample, o, d);
-            Hit h = trace_closest<WIDTH, MASK>(P.scene, o, d, 0.0f, tc);  // CPU preview: tnear 0
+            Hit h;
+            h.geom = MISS;
+            h.prim = 0;
+            if (!empty) {
+                camera_ray(P.cam, i, j, sample, o, d);
+                bool listed = false;
+                if constexpr (LISTS)
+                    listed = list_hit<MASK>(P, list, o, d, 0.0f, tc, h);
+                if (!listed)  // CPU preview: tnear 0
+                    h = trace_closest<WIDTH, MASK>(P.scene, o, d, 0.0f, tc);
+            }
             C3 c = P.bg;
             float a = P.bg_alpha;
             if (h.geom != MISS) {
@@ -942,7 +954,12 @@ void launch_path_primary_shade(const FrameParams& P, const PathState& S, cudaStr
     auto k = pick(P, k_path_primary_shade<2, MASK_SPHERES>, k_path_primary_shade<2, MASK_ALL>,
                   k_path_primary_shade<4, MASK_SPHERES>, k_path_primary_shade<4, MASK_ALL>);
     if (const int gk = grid_kind(P))
-        k = FR_GRID_KERNEL(k_path_primary_shade, gk);
+        k = P.lists ? (gk == 1   ? k_path_primary_shade<4, MASK_GRID, true>
+                       : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, true>
+                                 : k_path_primary_shade<4, MASK_GRID_PARTS_NO_MESH, true>)
+                    : FR_GRID_KERNEL(k_path_primary_shade, gk);
+    else if (P.lists)
+        k = k_path_primary_shade<4, MASK_SPHERES, true>;
     k<<<(n_items + 255) / 256, 256, 0, st>>>(P, S);
 }
 
@@ -1033,12 +1050,17 @@ void launch_histogram(const float4* linear, uint32_t n, uint32_t* counts, int nu
     k_histogram<<<blocks < cap ? (blocks ? blocks : 1u) : cap, 256, 0, st>>>(linear, n, counts);
 }
 
-void launch_preview(const FrameParams& P, uint32_t aa_n, uint2* hits, cudaStream_t st)
+bool preview_groups(const FrameParams& P, uint32_t aa_n)
 {
     // a group of 32 or 16 lanes per pixel when that divides the samples per pixel (with 2x2
     // anti-aliasing, 4 lanes per pixel were no faster than one thread on the 1M-sphere scene)
+    return P.preview_warp && (aa_n * aa_n) % 16u == 0u;
+}
+
+void launch_preview(const FrameParams& P, uint32_t aa_n, uint2* hits, cudaStream_t st)
+{
     const uint32_t ns = aa_n * aa_n;
-    if (P.preview_warp && ns % 16u == 0u) {
+    if (preview_groups(P, aa_n)) {
         const bool g32 = ns % 32u == 0u;
         const uint64_t threads = uint64_t(P.w) * P.h * (g32 ? 32u : 16u);
         auto k = g32 ? pick(P, k_preview_warp<2, MASK_SPHERES, 32>, k_preview_warp<2, MASK_ALL, 32>,
@@ -1052,6 +1074,17 @@ void launch_preview(const FrameParams& P, uint32_t aa_n, uint2* hits, cudaStream
                     : (gk == 1   ? k_preview_warp<4, MASK_GRID, 16>
                        : gk == 2 ? k_preview_warp<4, MASK_GRID_PARTS, 16>
                                  : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 16>);
+        if (P.lists) {
+            const int gk = grid_kind(P);
+            k = g32 ? (gk == 0   ? k_preview_warp<4, MASK_SPHERES, 32, true>
+                       : gk == 1 ? k_preview_warp<4, MASK_GRID, 32, true>
+                       : gk == 2 ? k_preview_warp<4, MASK_GRID_PARTS, 32, true>
+                                 : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 32, true>)
+                    : (gk == 0   ? k_preview_warp<4, MASK_SPHERES, 16, true>
+                       : gk == 1 ? k_preview_warp<4, MASK_GRID, 16, true>
+                       : gk == 2 ? k_preview_warp<4, MASK_GRID_PARTS, 16, true>
+                                 : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 16, true>);
+        }
         k<<<uint32_t((threads + 255u) / 256u), 256, 0, st>>>(P, aa_n, hits);
         return;
     }

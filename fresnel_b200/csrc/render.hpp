@@ -31,6 +31,9 @@ struct FrameParams {
     int preview_warp;        // 1: Preview with 32k samples per pixel traces one pixel per warp
     int refill_geom;         // -2: the scene's combined tree; >= 0: its one enabled geometry;
                              // -1: several per-geometry trees (refill not available)
+    const uint2* lists;      // per pixel, the primitives its camera rays can meet (beam.cuh);
+                             // null: every camera ray walks the acceleration structure
+    uint32_t list_enough;    // entries after which every list of a tile may end
     int highlight;
     C3 hl_color;
     float4* linear;     // [h][w] running mean, linear RGBA
@@ -93,6 +96,13 @@ void launch_path_bounce(const FrameParams& P, const PathState& S, int iteration,
 // The remaining bounces of every path in queue (iteration & 1) in one launch (k_path_tail).
 void launch_path_tail(const FrameParams& P, const PathState& S, int iteration,
                       const LaunchShape& shape, cudaStream_t st);
+// Per-pixel primitive lists of the frame's camera rays (beam.cuh: LIST_WORDS uint2 per pixel,
+// row by row), for scenes where lists are possible; lists_pay: `samples` camera rays per pixel are
+// expected to gain more than the lists cost.
+bool lists_possible(const FrameParams& P);
+bool lists_pay(const FrameParams& P, uint32_t samples);
+void launch_pixel_lists(const FrameParams& P, uint2* lists, cudaStream_t st);
+size_t pixel_list_words(const FrameParams& P);
 // ... then fold the batch's samples into each pixel's running mean, in sample order.
 void launch_path_fold(const FrameParams& P, const PathState& S, cudaStream_t st);
 // Diagnostic comparison of the two 4-wide traversal forms (sphere scenes).
@@ -103,6 +113,8 @@ void launch_traversal_compare(const SceneDev& sc, const float* rays, uint32_t n,
 constexpr uint32_t HIST_BINS = 512;
 void launch_histogram(const float4* linear, uint32_t n, uint32_t* counts, int num_sms,
                       cudaStream_t st);
+// Whether Preview traces a pixel's samples with a group of lanes.
+bool preview_groups(const FrameParams& P, uint32_t aa_n);
 // TracerDirect::render
 void launch_preview(const FrameParams& P, uint32_t aa_n, uint2* hits, cudaStream_t st);
 

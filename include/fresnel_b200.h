@@ -202,6 +202,12 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   pixel with a group of 32 lanes (8x8 anti-aliasing) or 16 (4x4), that many
  *                   of its samples at a time, summed in sample order; 0: one pixel per
  *                   thread.  The same outputs.
+ *   "pixel_lists"   camera rays take their closest hits from per-pixel lists of the primitives
+ *                   the pixel's beam can meet, built once per render, where the lists answer
+ *                   them: 0: never (every ray walks the acceleration structure); 1: for every
+ *                   scene traced through a grid or a tree over spheres; 2 (default): where
+ *                   they are expected to pay (at least 16 samples per pixel, 3 million camera
+ *                   rays, beams thinner than the primitives).  The same images in every case.
  *   "tail"          fused sphere-grid bounces: after this many bounce launches per wavefront
  *                   (0..64, default 1), one persistent launch follows every remaining path to
  *                   its end (a lane takes the next path once its own ends), with no queue

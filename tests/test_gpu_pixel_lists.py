@@ -1,0 +1,117 @@
+"""Per-pixel primitive lists (device option pixel_lists) against the walk they stand in for.
+
+A list may only answer a camera ray as the walk of the acceleration structure would, so every
+image must be the same bit for bit with the lists and without them, over every kind of structure,
+camera and primitive the lists take, and where they must decline: a camera among the primitives, a
+bounding radius smaller than the polyhedron, quaternions that are not of unit length.
+"""
+
+import math
+
+import numpy
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _spheres(dev, n=4000, box=22.0, camera="perspective", radii=0.5, f_stop=math.inf, at=None):
+    import fresnel_b200 as fresnel
+    rng = numpy.random.default_rng(3)
+    scene = fresnel.Scene(dev, lights=fresnel.light.cloudy())
+    pos = rng.uniform(-box / 2, box / 2, (n, 3)).astype(numpy.float32)
+    r = numpy.full(n, radii) if numpy.isscalar(radii) else rng.uniform(*radii, n)
+    g = fresnel.geometry.Sphere(scene, position=pos, radius=r.astype(numpy.float32),
+                                outline_width=0.05)
+    g.color[:] = rng.uniform(0, 1, (n, 3))
+    g.material = fresnel.material.Material(primitive_color_mix=1.0, roughness=0.4)
+    where = numpy.array((1.1 * box, 0.8 * box, 1.3 * box) if at is None else at, float)
+    if camera == "perspective":
+        d = float(numpy.linalg.norm(where))
+        scene.camera = fresnel.camera.Perspective(position=where, look_at=(0, 0, 0), up=(0, 1, 0),
+                                                  focal_length=0.25 * d, focus_distance=d,
+                                                  f_stop=f_stop, height=0.3 * box)
+    else:
+        scene.camera = fresnel.camera.Orthographic(position=where, look_at=(0, 0, 0),
+                                                   up=(0, 1, 0), height=1.3 * box)
+    return scene
+
+
+def _cubes(dev, radius=None, scale=1.0):
+    """Cubes and bonds; radius: the stated bounding radius, scale: the quaternions' length."""
+    import fresnel_b200 as fresnel
+    from fresnel_b200 import workloads
+    rng = numpy.random.default_rng(8)
+    scene = fresnel.Scene(dev, lights=fresnel.light.rembrandt())
+    info = workloads.unit_cube_planes()
+    if radius is not None:
+        info["radius"] = radius
+    pos = rng.uniform(-7, 7, (500, 3)).astype(numpy.float32)
+    fresnel.geometry.ConvexPolyhedron(scene, info, position=pos, color=(0.7, 0.4, 0.2),
+                                      orientation=workloads.random_quaternions(rng, 500) * scale,
+                                      outline_width=0.03)
+    pts = numpy.stack([pos[:200], pos[200:400]], axis=1) * 0.5
+    fresnel.geometry.Cylinder(scene, points=pts, radius=0.1, color=(0.2, 0.3, 0.8))
+    scene.camera = fresnel.camera.Orthographic.fit(scene)
+    return scene
+
+
+def _mixed(dev):
+    from fresnel_b200 import workloads
+    return workloads.config3(dev, scale=0.004)
+
+
+def _layers(dev):
+    from fresnel_b200 import workloads
+    return workloads.polygons(dev, nx=12, ny=9, spheres=150)
+
+
+SCENES = {
+    "grid": (_spheres, {}),
+    "grid_ortho": (_spheres, dict(camera="orthographic")),
+    "grid_lens": (_spheres, dict(f_stop=4.0)),
+    "grid_radii": (_spheres, dict(radii=(0.02, 1.5), n=1500)),
+    "grid_inside": (_spheres, dict(at=(0.3, 0.2, 0.4))),
+    "grid_distant": (_spheres, dict(at=(900.0, 0.0, 10.0))),
+    "grid_one": (_spheres, dict(n=1)),
+    "tree": (_spheres, dict(accel=0)),
+    "tree_lens": (_spheres, dict(accel=0, f_stop=8.0, radii=(0.02, 1.5))),
+    "tree_ortho": (_spheres, dict(accel=0, camera="orthographic")),
+    "mixed": (_mixed, {}),
+    "layers": (_layers, {}),
+    "cubes": (_cubes, {}),
+    "cubes_small_radius": (_cubes, dict(radius=0.4)),
+    "cubes_scaled": (_cubes, dict(scale=1.4)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+@pytest.mark.parametrize("size", [(97, 61), (8, 4), (33, 1)])
+def test_lists_give_the_walks_images(gpu_device, name, size):
+    import fresnel_b200 as fresnel
+    make, args = SCENES[name]
+    args = dict(args)
+    option = gpu_device._device.setOption
+    option("accel", args.pop("accel", 2))
+    try:
+        scene = make(gpu_device, **args)
+        images = []
+        for lists in (0, 1):
+            option("pixel_lists", lists)
+            path = fresnel.tracer.Path(gpu_device, *size)
+            path.seed = 11
+            path.sample(scene, 40)
+            preview = fresnel.tracer.Preview(gpu_device, *size, anti_alias=True)
+            preview.seed = 5
+            preview.render(scene)
+            images.append((path.linear_output[:], preview.linear_output[:], path._tracer.getStats()))
+    finally:
+        option("pixel_lists", 2)
+        option("accel", 2)
+    numpy.testing.assert_array_equal(images[0][0].view(numpy.uint32),
+                                     images[1][0].view(numpy.uint32))
+    numpy.testing.assert_array_equal(images[0][1].view(numpy.uint32),
+                                     images[1][1].view(numpy.uint32))
+    for key in ("rays", "paths"):
+        assert images[0][2][key] == images[1][2][key]
+    if name in ("grid", "tree") and size == (97, 61):  # the lists are in use
+        assert images[1][2]["box_tests"] < 0.8 * images[0][2]["box_tests"]
