@@ -89,6 +89,7 @@ struct PathBuffers {
     DevArray<float4> prim_o, prim_d, ray_o, ray_d, att, result, sample;
     DevArray<uint2> prim_hit, ls_depth, hit;
     DevArray<uint32_t> q0, q1, ctr;
+    DevArray<float4> rec_o, rec_d, rec_a;  // see reserve_records
     // slots for n paths; `moved` is set when an array changed address
     cudaError_t reserve(size_t n, bool* moved = nullptr)
     {
@@ -122,7 +123,17 @@ struct PathBuffers {
                     *moved = true;
         return e;
     }
-    PathState state() const
+    // room for the second packed queue beside several light samples per camera ray
+    cudaError_t reserve_records(size_t n)
+    {
+        cudaError_t e = rec_o.reserve(n);
+        if (e == cudaSuccess)
+            e = rec_d.reserve(n);
+        if (e == cudaSuccess)
+            e = rec_a.reserve(n);
+        return e;
+    }
+    PathState state(bool lights = false) const
     {
         PathState S;
         S.prim_o = prim_o.ptr;
@@ -138,6 +149,14 @@ struct PathBuffers {
         S.queue[0] = q0.ptr;
         S.queue[1] = q1.ptr;
         S.ctr = ctr.ptr;
+        // packed queues: the second one in the arrays that only several light samples per camera
+        // ray use, or in arrays of its own (reserve_records)
+        S.rec_o[0] = ray_o.ptr;
+        S.rec_d[0] = ray_d.ptr;
+        S.rec_a[0] = att.ptr;
+        S.rec_o[1] = lights ? rec_o.ptr : prim_o.ptr;
+        S.rec_d[1] = lights ? rec_d.ptr : prim_d.ptr;
+        S.rec_a[1] = lights ? rec_a.ptr : result.ptr;
         return S;
     }
 };
@@ -168,6 +187,8 @@ struct fr_device {
                                            // 0 never, 1 whenever possible, 2 where they pay
     DevArray<uint2> lists;                 // those of the render in progress
     int accel = 2;                         // sphere grid: 0 never, 1 whenever possible, 2 auto
+    int wave = 1;                          // extension rays over packed queues
+    cudaEvent_t wave_ev[2] = {nullptr, nullptr};  // their queue lengths are read back
     int fuse_shade = 1;                    // primary rays shaded in the primary pass
     int tail_after = 1;                    // fused bounce launches before the tail kernel (-1: none)
     float grid_cells_per_prim = 1.5f;      // grid cells per sphere
@@ -991,6 +1012,13 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
     return P;
 }
 
+// Path slots from which extension rays go over packed queues (below, the launches cost more than
+// the fused bounce and tail kernels lose: frames of 2M slots and few hits 0.90-0.96x), and the
+// queue length below which the tail kernel follows the remaining paths (200k spheres 1024x768, 16
+// samples: 3.14 ms at 16k, 2.96 at 256k, 2.65 at 1.5M; 1M spheres 1080p: 46.3, 45.2, 44.6 ms).
+constexpr size_t WAVE_MIN_SLOTS = 1u << 21;
+constexpr uint32_t WAVE_TAIL_RAYS = 3u << 19;
+
 // Builds the frame's pixel lists on the stream and puts them into P where they apply and
 // `samples` camera rays per pixel pay for them.
 void prepare_lists(fr_device* dev, FrameParams& P, uint32_t samples)
@@ -1162,6 +1190,8 @@ fr_status fr_device_create(int n, fr_device** out)
         e = cudaMemset(d->status.ptr, 0, sizeof(uint32_t));
     if (e == cudaSuccess)
         e = cudaMallocHost((void**)&d->h_count, 4 * sizeof(uint32_t));
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+        e = cudaEventCreateWithFlags(&d->wave_ev[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete d;
         return cuda_fail(e, "creating the device");
@@ -1184,6 +1214,9 @@ fr_status fr_device_destroy(fr_device* d)
     for (int k = 0; k < 2; ++k)
         if (d->timer[k])
             cudaEventDestroy(d->timer[k]);
+    for (int k = 0; k < 2; ++k)
+        if (d->wave_ev[k])
+            cudaEventDestroy(d->wave_ev[k]);
     if (d->h_count)
         cudaFreeHost(d->h_count);
     delete d;
@@ -1296,6 +1329,10 @@ fr_status fr_device_set_option(fr_device* d, const char* name, double value)
         if (value != 0.0 && value != 1.0)
             return fail(FR_ERR_INVALID, "preview_warp must be 0 or 1");
         d->preview_warp = int(value);
+    } else if (n == "wave") {
+        if (value != 0.0 && value != 1.0)
+            return fail(FR_ERR_INVALID, "wave must be 0 or 1");
+        d->wave = int(value);
     } else if (n == "pixel_lists") {
         if (value != 0.0 && value != 1.0 && value != 2.0)
             return fail(FR_ERR_INVALID, "pixel_lists must be 0 (never), 1 or 2 (where they pay)");
@@ -1346,6 +1383,8 @@ fr_status fr_device_get_option(const fr_device* d, const char* name, double* val
         *value = d->tail_after;
     else if (n == "preview_warp")
         *value = d->preview_warp;
+    else if (n == "wave")
+        *value = d->wave;
     else if (n == "pixel_lists")
         *value = d->pixel_lists;
     else if (n == "fuse_shade")
@@ -1849,7 +1888,17 @@ fr_status fr_tracer_render_path(fr_tracer* t, fr_scene* sc, const fr_render_para
         return s;
     FrameParams P = frame_params(t, sc, p, false, 1);
     P.light_samples = light_samples;
-    PathState S = t->dev->path.state();
+    // extension rays over packed queues (wave.cu)
+    bool wave = t->dev->wave && t->dev->fuse_shade == 1 && t->dev->tail_after >= 0 && !P.refill &&
+                !P.packet && P.scene.grid.n_cells != 0 && !P.scene.grid.parts &&
+                padded_pixels(t->w, t->h, t->dev->tile_log2) * batch >= WAVE_MIN_SLOTS;
+    if (wave && light_samples > 1 &&
+        t->dev->path.reserve_records(padded_pixels(t->w, t->h, t->dev->tile_log2) * batch) !=
+            cudaSuccess) {
+        cudaGetLastError();  // the fused bounces need no second queue of records
+        wave = false;
+    }
+    PathState S = t->dev->path.state(wave && light_samples > 1);
     t->dev->path_owner = t;
     cudaStream_t st = t->dev->stream;
     FR_CUDA(cudaMemsetAsync(S.ctr, 0, 4 * sizeof(uint32_t), st), "clearing queue lengths");
@@ -1876,13 +1925,42 @@ fr_status fr_tracer_render_path(fr_tracer* t, fr_scene* sc, const fr_render_para
         P.batch = batch < n_render - done ? batch : n_render - done;
         if (fused) {
             FR_CUDA(cudaMemsetAsync(S.ctr, 0, 4 * sizeof(uint32_t), st), "clearing the queues");
-            timed(0, [&] { launch_path_primary_shade(P, S, st); });
+            timed(0, [&] { launch_path_primary_shade(P, S, wave, st); });
         } else {
             FR_CUDA(cudaMemsetAsync(S.ctr + 3, 0, sizeof(uint32_t), st), "clearing a counter");
             timed(0, [&] { launch_path_primary(P, S, t->dev->shape, st); });
         }
         t->launches++;
         int it = 0;
+        if (wave) {
+            // trace and shade queue it & 1 while it is long; its length is read back while its
+            // own pass runs, so that the host never holds the stream up
+            uint32_t* len = t->dev->h_count + 1;
+            while (true) {
+                const int w = it & 1;
+                FR_CUDA(cudaMemcpyAsync(len + w, S.ctr + w, sizeof(uint32_t),
+                                        cudaMemcpyDeviceToHost, st),
+                        "reading the queue length");
+                FR_CUDA(cudaEventRecord(t->dev->wave_ev[w], st), "path tracer");
+                timed(2, [&] { launch_wave_trace(P, S, w, t->dev->shape, st); });
+                timed(1, [&] { launch_wave_shade(P, S, w, t->dev->shape, st); });
+                t->launches += 2;
+                FR_CUDA(cudaGetLastError(), "launching the path tracer");
+                ++it;
+                FR_CUDA(cudaEventSynchronize(t->dev->wave_ev[w]), "path tracer");
+                if (len[w] < WAVE_TAIL_RAYS || it >= MAX_ITER)
+                    break;
+            }
+            timed(2, [&] { launch_wave_tail(P, S, it & 1, t->dev->shape, st); });
+            t->launches += 1;
+            FR_CUDA(cudaGetLastError(), "launching the path tracer");
+            launch_path_fold(P, S, st);
+            t->launches++;
+            t->dev->path_k = P.batch;
+            t->dev->path_tile_log2 = P.tile_log2;
+            done += P.batch;
+            continue;
+        }
         // bounces fused too: by default for sphere-grid scenes only (a BVH walk in a kernel
         // compiled for 3 blocks per SM is slower than the separate passes)
         const bool bounces =

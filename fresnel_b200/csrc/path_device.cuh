@@ -171,10 +171,58 @@ __device__ __forceinline__ void shade_load(const FrameParams& P, const PathState
     L.have_sf = false;
 }
 
+// After a vertex: store the continuing path (or leave it to the caller: REC), or move to the next
+// light sample from the cached primary hit, or store the finished pixel sample
+// (fresnel/cpu/TracerPath.cc:228: radiance / L, alpha).
+template <bool REC>
+__device__ __forceinline__ ShadeStep shade_end(const FrameParams& P, const PathState& S,
+                                               ShadeLane& L)
+{
+    PathS& s = L.s;
+    const uint32_t p = L.p;
+    if (!s.done) {
+        s.depth += 1u;
+        if constexpr (REC) {
+            if (P.light_samples > 1u)
+                st_cs(S.result + (p), f4(s.result));
+        } else {
+            st_cs(S.ray_o + (p), f4(s.origin));
+            st_cs(S.ray_d + (p), f4(s.dir));
+            st_cs(S.att + (p), f4(s.att));
+            st_cs(S.result + (p), f4(s.result));
+            st_cs(S.ls_depth + (p), make_uint2(L.ls, s.depth));
+        }
+        return STEP_CONTINUE;
+    }
+    if (L.ls + 1u < P.light_samples) {
+        ++L.ls;
+        if (s.depth == 0) {  // the next light sample starts from this same vertex
+            L.have_sf = true;
+        } else {
+            L.ro = xyz(ld_cs(S.prim_o + (p)));
+            L.rd = xyz(ld_cs(S.prim_d + (p)));
+            L.h = REC ? ld_cs(S.prim_hit + (p)) : L.ph;
+            L.have_sf = false;
+        }
+        s.depth = 0;
+        s.att = c3(1.0f, 1.0f, 1.0f);
+        return STEP_RESTART;
+    }
+    C3 out = c_div_recip(s.result, float(P.light_samples));
+    // (a record's path began at a hit)
+    st_cs(S.sample + (p),
+          make_float4(out.r, out.g, out.b, (!REC && L.ph.x == MISS) ? P.bg_alpha : 1.0f));
+    return STEP_FINISHED;
+}
+
 // Shade the lane's current vertex (TracerPath's hit/miss programs,
 // fresnel/common/TracerPathMethods.h:36-168, light samples in order), then store the continuing
 // path, or move to the next light sample from the cached primary hit, or store the finished
 // pixel sample (fresnel/cpu/TracerPath.cc:228: radiance / L, alpha).
+//
+// REC: the path's state travels in a packed queue's record (wave.cu), which the caller writes; with
+// several light samples per slot their radiance so far stays with the slot.
+template <bool REC = false>
 __device__ __forceinline__ ShadeStep shade_step(const FrameParams& P, const PathState& S,
                                                 ShadeLane& L)
 {
@@ -194,41 +242,24 @@ __device__ __forceinline__ ShadeStep shade_step(const FrameParams& P, const Path
     } else {
         path_miss_lights(s, P.lights, L.rd);
     }
-    const uint32_t p = L.p;
-    if (!s.done) {
-        s.depth += 1u;
-        st_cs(S.ray_o + (p), f4(s.origin));
-        st_cs(S.ray_d + (p), f4(s.dir));
-        st_cs(S.att + (p), f4(s.att));
-        st_cs(S.result + (p), f4(s.result));
-        st_cs(S.ls_depth + (p), make_uint2(L.ls, s.depth));
-        return STEP_CONTINUE;
-    }
-    if (L.ls + 1u < P.light_samples) {
-        ++L.ls;
-        if (s.depth == 0) {  // the next light sample starts from this same vertex
-            L.have_sf = true;
-        } else {
-            L.ro = xyz(ld_cs(S.prim_o + (p)));
-            L.rd = xyz(ld_cs(S.prim_d + (p)));
-            L.h = L.ph;
-            L.have_sf = false;
-        }
-        s.depth = 0;
-        s.att = c3(1.0f, 1.0f, 1.0f);
-        return STEP_RESTART;
-    }
-    C3 out = c_div_recip(s.result, float(P.light_samples));
-    st_cs(S.sample + (p), make_float4(out.r, out.g, out.b, L.ph.x == MISS ? P.bg_alpha : 1.0f));
-    return STEP_FINISHED;
+    return shade_end<REC>(P, S, L);
+}
+
+// A record's ray that met nothing: the lights it sees, then the end of its light sample; true when
+// the lane now holds the next one's first vertex.
+__device__ __forceinline__ bool shade_miss(const FrameParams& P, const PathState& S, ShadeLane& L)
+{
+    path_miss_lights(L.s, P.lights, L.rd);
+    return shade_end<true>(P, S, L) == STEP_RESTART;
 }
 
 // Shade a lane until its path needs another closest hit (returns true) or its pixel sample is
 // finished (returns false).
+template <bool REC = false>
 __device__ __forceinline__ bool shade_run(const FrameParams& P, const PathState& S, ShadeLane& L)
 {
     while (true) {
-        const ShadeStep r = shade_step(P, S, L);
+        const ShadeStep r = shade_step<REC>(P, S, L);
         if (r != STEP_RESTART)
             return r == STEP_CONTINUE;
     }
@@ -280,9 +311,11 @@ __device__ __forceinline__ bool primary_ray(const FrameParams& P, const PathStat
 // storing the primary ray (unless a later light sample restarts from it) or reading anything
 // back.  Returns true when the path continues (its extension ray is stored; queue it).
 // LISTS: the frame has pixel lists (beam.cuh).
-template <int WIDTH, uint32_t MASK, bool LISTS = false>
+// REC: the continuing path is left in L for the caller to queue as a packed record.
+template <int WIDTH, uint32_t MASK, bool LISTS = false, bool REC = false>
 __device__ __forceinline__ bool primary_shade(const FrameParams& P, const PathState& S,
-                                              const PrimaryItem& it, uint32_t slot, TraceCount& tc)
+                                              const PrimaryItem& it, uint32_t slot, TraceCount& tc,
+                                              ShadeLane& L)
 {
     V3 o, d;
     Hit h;
@@ -311,7 +344,6 @@ __device__ __forceinline__ bool primary_shade(const FrameParams& P, const PathSt
         st_cs(S.prim_o + (slot), f4(o));
         st_cs(S.prim_d + (slot), f4(d));
     }
-    ShadeLane L;
     L.p = slot;
     L.pixel = it.j * P.w + it.i;
     L.n_samples = P.n_samples + it.k;
@@ -326,7 +358,25 @@ __device__ __forceinline__ bool primary_shade(const FrameParams& P, const PathSt
     L.ro = o;
     L.rd = d;
     L.have_sf = false;
-    return shade_run(P, S, L);
+    return shade_run<REC>(P, S, L);
+}
+
+template <int WIDTH, uint32_t MASK>
+__device__ __forceinline__ bool primary_shade(const FrameParams& P, const PathState& S,
+                                              const PrimaryItem& it, uint32_t slot, TraceCount& tc)
+{
+    ShadeLane L;
+    return primary_shade<WIDTH, MASK, false, false>(P, S, it, slot, tc, L);
+}
+
+// The lane's continuing path as record i of packed queue q.
+__device__ __forceinline__ void store_record(const PathState& S, int q, uint32_t i,
+                                             const ShadeLane& L)
+{
+    const PathS& s = L.s;
+    st_cs(S.rec_o[q] + i, make_float4(s.origin.x, s.origin.y, s.origin.z, __uint_as_float(L.p)));
+    st_cs(S.rec_d[q] + i, make_float4(s.dir.x, s.dir.y, s.dir.z, __uint_as_float(s.depth)));
+    st_cs(S.rec_a[q] + i, make_float4(s.att.r, s.att.g, s.att.b, __uint_as_float(L.ls)));
 }
 
 // Extension ray of slot p traced and its hit shaded at once (a bounce): the path state is read as
@@ -367,11 +417,12 @@ __device__ __forceinline__ bool bounce(const FrameParams& P, const PathState& S,
 // (frame 75.0 -> 64.8 ms).  push_block and flush_block share them over a block.
 constexpr uint32_t PATH_BLOCK = 256;  // threads per block of every kernel using them
 
-// Append the slots of the block's threads with push set to queue q, in thread order, with one
-// atomic, and add the block's traversal counts to counters[0] (box tests) and counters[1]
+// Places in queue q for the block's threads with push set, in thread order, taken with one
+// atomic (the thread's own is returned), and add the block's traversal counts to counters[0] (box tests) and counters[1]
 // (primitive tests).  Every thread of the block calls it (once per kernel).
-__device__ __forceinline__ void push_block(const PathState& S, int q, bool push, uint32_t slot,
-                                           const TraceCount& tc, unsigned long long* counters)
+__device__ __forceinline__ uint32_t push_block(const PathState& S, int q, bool push,
+                                               const TraceCount& tc,
+                                               unsigned long long* counters)
 {
     constexpr uint32_t W = PATH_BLOCK / 32;
     __shared__ uint32_t at[W], box[W], prim[W];
@@ -407,8 +458,7 @@ __device__ __forceinline__ void push_block(const PathState& S, int q, bool push,
         }
     }
     __syncthreads();
-    if (push)
-        st_cs(S.queue[q] + (at[warp] + __popc(m & ((1u << lane) - 1u))), slot);
+    return at[warp] + __popc(m & ((1u << lane) - 1u));
 }
 
 // Add the block's traversal counts to the counters alone (any block shape).

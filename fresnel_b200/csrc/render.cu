@@ -66,7 +66,9 @@ __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S
         slot = g;
         push = primary_ray<WIDTH, MASK>(P, S, it, slot, tc);
     }
-    push_block(S, 1, push, slot, tc, P.stats + 3);
+    const uint32_t at = push_block(S, 1, push, tc, P.stats + 3);
+    if (push)
+        st_cs(S.queue[1] + at, slot);
     count_primary(P, g);
 }
 
@@ -75,7 +77,8 @@ __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S
 // frame's first shade pass is not launched.  Limited to fused_blocks<MASK> blocks of 256 threads
 // per SM.  LISTS: the frame has pixel lists (a kernel of its own, so that frames without them
 // carry none of their code: path images of polygons 3% faster).
-template <int WIDTH, uint32_t MASK, bool LISTS = false>
+// REC: continuing paths as packed records (wave.cu).
+template <int WIDTH, uint32_t MASK, bool LISTS = false, bool REC = false>
 __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(FrameParams P, PathState S)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -84,11 +87,18 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(
     it.valid = false;
     if (g < n_items)
         it = primary_item(g, P.w, P.h, P.batch, P.tile_log2);
+    ShadeLane L;
     bool push = false;
     TraceCount tc;
     if (it.valid)
-        push = primary_shade<WIDTH, MASK, LISTS>(P, S, it, g, tc);
-    push_block(S, 0, push, g, tc, P.stats + 3);
+        push = primary_shade<WIDTH, MASK, LISTS, REC>(P, S, it, g, tc, L);
+    const uint32_t at = push_block(S, 0, push, tc, P.stats + 3);
+    if (push) {
+        if constexpr (REC)
+            store_record(S, 0, at, L);
+        else
+            st_cs(S.queue[0] + at, g);
+    }
     count_primary(P, g);
 }
 
@@ -881,6 +891,7 @@ template <class K> int blocks_per_sm(K kernel)
 LaunchShape path_launch_shape(int num_sms)
 {
     LaunchShape s;
+    wave_launch_shape(num_sms, s);
     s.shade_grid = num_sms * blocks_per_sm(k_path_shade<>);
     s.shade_grid_occ[0] = num_sms * blocks_per_sm(k_path_shade<3>);
     s.refill_grid[0] = num_sms * blocks_per_sm(k_path_extend_refill<MASK_SPHERES>);
@@ -948,12 +959,16 @@ void launch_path_primary(const FrameParams& P, const PathState& S, const LaunchS
     k<<<(n_items + 255) / 256, 256, 0, st>>>(P, S);
 }
 
-void launch_path_primary_shade(const FrameParams& P, const PathState& S, cudaStream_t st)
+void launch_path_primary_shade(const FrameParams& P, const PathState& S, bool rec, cudaStream_t st)
 {
     const uint32_t n_items = primary_items(P.w, P.h, P.batch, P.tile_log2);
     auto k = pick(P, k_path_primary_shade<2, MASK_SPHERES>, k_path_primary_shade<2, MASK_ALL>,
                   k_path_primary_shade<4, MASK_SPHERES>, k_path_primary_shade<4, MASK_ALL>);
-    if (const int gk = grid_kind(P))
+    const int gk = grid_kind(P);
+    if (rec && gk == 1)
+        k = P.lists ? k_path_primary_shade<4, MASK_GRID, true, true>
+                    : k_path_primary_shade<4, MASK_GRID, false, true>;
+    else if (gk)
         k = P.lists ? (gk == 1   ? k_path_primary_shade<4, MASK_GRID, true>
                        : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, true>
                                  : k_path_primary_shade<4, MASK_GRID_PARTS_NO_MESH, true>)

@@ -55,10 +55,18 @@ struct PathState {
     uint2* hit;         // closest hit of the last extension ray
     float4* sample;     // the finished pixel sample of each slot (folded in order at the end)
     uint32_t* queue[2];
+    // Packed queues (wave.cu): record i of queue q is (ray origin, slot), (ray direction, depth),
+    // (throughput, light sample) in rec_o[q][i], rec_d[q][i], rec_a[q][i], its hit hit[i].
+    float4* rec_o[2];
+    float4* rec_d[2];
+    float4* rec_a[2];
     uint32_t* ctr;      // [0], [1] queue lengths, [2] extend and [3] primary work counters
 };
 
 struct LaunchShape {
+    int trace_grid[3];       // packed queues: trace, shade and tail kernels, per grid kind
+    int shade_rec_grid[3];   // [sphere grid|parts grid|parts grid without meshes]
+    int tail_rec_grid[3];
     int shade_grid;
     int shade_grid_occ[2];   // shade kernel compiled for 3|4 blocks per SM
     int refill_grid[2];      // extension kernel with per-lane refill [spheres only|all types]
@@ -87,7 +95,7 @@ void launch_path_extend(const FrameParams& P, const PathState& S, int iteration,
 // Or, instead of the primary pass and the first shade pass: primary rays shaded at once, the
 // continuing paths in queue 0 (all four counters must be zero); the loop then starts with the
 // extend of iteration 0.
-void launch_path_primary_shade(const FrameParams& P, const PathState& S, cudaStream_t st);
+void launch_path_primary_shade(const FrameParams& P, const PathState& S, bool rec, cudaStream_t st);
 // With the primary pass shaded at once, iteration i may instead be one fused bounce: the rays of
 // q[i&1] traced and shaded, continuing paths into q[(i&1)^1] (whose length and ctr[2] must be
 // zero).
@@ -103,6 +111,17 @@ bool lists_possible(const FrameParams& P);
 bool lists_pay(const FrameParams& P, uint32_t samples);
 void launch_pixel_lists(const FrameParams& P, uint2* lists, cudaStream_t st);
 size_t pixel_list_words(const FrameParams& P);
+// With the primary pass shaded at once over packed queues (records of the continuing paths in queue
+// 0; `rec` below): the hits of queue q's rays, then their shading into queue q ^ 1 (whose length
+// the trace clears, as the shading clears the work counter of the next trace), and in the end the
+// remaining bounces of every path in queue q.
+void wave_launch_shape(int num_sms, LaunchShape& shape);
+void launch_wave_trace(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
+                       cudaStream_t st);
+void launch_wave_shade(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
+                       cudaStream_t st);
+void launch_wave_tail(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
+                      cudaStream_t st);
 // ... then fold the batch's samples into each pixel's running mean, in sample order.
 void launch_path_fold(const FrameParams& P, const PathState& S, cudaStream_t st);
 // Diagnostic comparison of the two 4-wide traversal forms (sphere scenes).

@@ -208,6 +208,10 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   scene traced through a grid or a tree over spheres; 2 (default): where
  *                   they are expected to pay (at least 16 samples per pixel, 3 million camera
  *                   rays, beams thinner than the primitives).  The same images in every case.
+ *   "wave"          1 (default): bounces of scenes traced through a sphere grid trace and shade in
+ *                   separate passes over queues of whole path records (at least 2M path
+ *                   slots), the tracing with per-lane refill; 0: fused bounces as below.  The
+ *                   same images in both cases.
  *   "tail"          fused sphere-grid bounces: after this many bounce launches per wavefront
  *                   (0..64, default 1), one persistent launch follows every remaining path to
  *                   its end (a lane takes the next path once its own ends), with no queue
