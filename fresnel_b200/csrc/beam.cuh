@@ -1,7 +1,7 @@
 // beam.cuh -- per-pixel lists of the primitives a pixel's camera rays can meet.
 //
 // The camera rays of one pixel (its anti-aliasing or Monte Carlo samples) form a thin beam: all of
-// them meet the same few primitives.  k_pixel_lists_grid and k_pixel_lists_bvh (lists.cu) walks the acceleration structure
+// them meet the same few primitives.  k_pixel_lists_grid (lists.cu) walks the acceleration structure
 // once per beam and stores, per pixel, the primitives some ray of the beam may hit, nearest first,
 // and a depth up to which that list is complete; list_hit then finds a sample's closest hit by
 // testing the listed primitives alone, with the tests and the acceptance rule of the structure's
@@ -24,7 +24,7 @@ namespace fr {
 
 // A pixel's list: LIST_WORDS uint2; word 0 is (entries, bits of the complete distance), the
 // others (slot, bits of the nearest distance a ray can be hit at).  Slots number the grid's
-// references or the tree's leaf slots.  128 bytes: one line per pixel.
+// references.  128 bytes: one line per pixel.
 constexpr uint32_t LIST_WORDS = 16;
 constexpr uint32_t LIST_MAX = LIST_WORDS - 1;
 
@@ -45,7 +45,7 @@ __device__ __forceinline__ bool hit_inside_box(const SceneDev& sc, const Hit& h,
     auto in3 = [&](V3 c, float r) {
         return fmaxf(fmaxf(fabsf(x.x - c.x), fabsf(x.y - c.y)), fabsf(x.z - c.z)) <= r - m;
     };
-    if constexpr ((MASK & MASK_ALL) == 0u || (MASK & MASK_ALL) == MASK_SPHERES) {
+    if constexpr ((MASK & MASK_ALL) == 0u) {
         return in3(load3(g.position, h.prim), __ldg(g.radius + h.prim));
     } else {
         if (g.type == FR_GEOM_SPHERE)
@@ -111,7 +111,7 @@ __device__ __forceinline__ bool list_hit(const FrameParams& P, const uint2* list
             return complete == __int_as_float(0x7f800000);
         h.geom = G.geom;
         h.prim = __ldg(G.ref_prim + slot);
-    } else if constexpr ((MASK & MASK_GRID) != 0u) {
+    } else {
         const RayK ray = make_rayk(o, d);
         uint32_t hg = MISS, hp = 0, last_g = MISS, last_p = 0;
         for (uint32_t e = 1; e <= head.x; ++e) {
@@ -125,23 +125,6 @@ __device__ __forceinline__ bool list_hit(const FrameParams& P, const uint2* list
             return complete == __int_as_float(0x7f800000);
         h.geom = hg;
         h.prim = hp;
-    } else {  // trees over spheres
-        const RayK ray = make_rayk(o, d);
-        uint32_t hg = MISS, slot = 0;
-        for (uint32_t e = 1; e <= head.x; ++e) {
-            const uint2 c = __ldg(list + e);
-            if (tmax < __uint_as_float(c.y))
-                break;
-            if (P.refill_geom == -2)
-                leaf_test_mixed<MASK_SPHERES>(sc, ray, c.x, 1u, tnear, tmax, hg, slot, tc);
-            else
-                leaf_test<FR_GEOM_SPHERE>(sc.geoms[P.refill_geom], uint32_t(P.refill_geom), ray,
-                                          c.x, 1u, tnear, tmax, hg, slot, tc);
-        }
-        if (hg == MISS)
-            return complete == __int_as_float(0x7f800000);
-        h.geom = hg;
-        h.prim = __ldg((P.refill_geom == -2 ? sc.order : sc.geoms[hg].order) + slot);
     }
     return tmax < complete && hit_inside_box<MASK>(sc, h, o, d, tmax);
 }

@@ -5,7 +5,6 @@
 // beam by all lanes side by side (one reference per lane), and each survivor is then tested by
 // every lane against its own pixel's beam and kept in the lane's list.  One walk serves 32 pixels
 // and all their samples: on the 1M-sphere frame at 1920x1080 the lists of a frame take about 0.5 ms.
-// Trees over spheres: one thread per pixel walks the 4-wide tree with boxes widened by its beam.
 //
 // A beam is an axis (o, d) and a radius R(tau) about the axis point at distance tau that covers
 // every ray of the beam at the same parameter: the jitter (perspective: growing with tau;
@@ -487,148 +486,6 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
         L.store(out + size_t(LIST_WORDS) * (size_t(j) * P.w + i));
 }
 
-// Nodes a pixel's walk of a tree visits at most: a thin beam needs some 20 to 40; one that is as
-// wide as the spheres it runs through (a dense droplet seen from afar) would visit hundreds for a
-// list that few of its rays can use.
-constexpr uint32_t LIST_VISITS = 96;
-
-// Lists over a 4-wide tree of spheres (a combined tree, or the scene's one geometry's tree).
-__global__ void __launch_bounds__(128) k_pixel_lists_bvh(FrameParams P, uint2* out)
-{
-    __shared__ uint2 entries[4][LIST_MAX * 32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t tiles_x = (P.w + 7u) >> 3;
-    const uint32_t tile = blockIdx.x * 4u + warp;
-    const uint32_t ty = tile / tiles_x, tx = tile - ty * tiles_x;
-    const uint32_t i = tx * 8u + (lane & 7u), j = ty * 4u + (lane >> 3);
-    if (i >= P.w || j >= P.h)
-        return;
-    const SceneDev& sc = P.scene;
-    const bool combined = P.refill_geom == -2;
-    const GeomDev& g = sc.geoms[combined ? 0 : P.refill_geom];
-    const float4* nodes4 = combined ? sc.nodes4 : g.nodes4;
-    const uint32_t n_nodes4 = combined ? sc.n_nodes4 : g.n_nodes4;
-    const uint32_t n_prims = combined ? sc.n_prims : g.n_prims;
-    ListBuilder L;
-    L.start(entries[warp] + lane);
-    uint2* const to = out + size_t(LIST_WORDS) * (size_t(j) * P.w + i);
-    Beam b = make_beam(P.cam, float(i) + 0.5f, float(j) + 0.5f, PIXEL_REACH);
-    // the root's box: the farthest point and the size of the coordinates
-    float far = 0.0f, scale = 0.0f;
-    if (n_nodes4) {
-        const float* f = reinterpret_cast<const float*>(nodes4);
-        const uint32_t* cc = reinterpret_cast<const uint32_t*>(nodes4 + 7);
-        float far2 = 0.0f;
-        for (int c = 0; c < 4; ++c) {
-            if (__ldg(cc + c) == EMPTY_CHILD)
-                continue;
-            float s = 0.0f;
-            for (int k = 0; k < 3; ++k) {
-                const float lo = __ldg(f + 8 * k + c), hi = __ldg(f + 8 * k + 4 + c);
-                const float e = fmaxf(fabsf(lo - comp(b.o, k)), fabsf(hi - comp(b.o, k)));
-                s += e * e;
-                scale = fmaxf(scale, fmaxf(fabsf(lo), fabsf(hi)));
-            }
-            far2 = fmaxf(far2, s);
-        }
-        far = root(far2) * (1.0f + 1e-5f);
-    }
-    if (!(finish_beam(b, far) && far <= 16.0f * scale)) {
-        L.complete = n_nodes4 ? 0.0f : INF;
-        L.store(to);
-        return;
-    }
-    const RayK ray = make_rayk(b.o, b.d);
-    const float R = b.over(0.0f, far * (1.0f + 2.0f * b.g));
-    const float back = (1.0f - b.g) * (1.0f - 1e-5f);  // box entry along the axis -> t
-    uint32_t stack_node[TRAVERSAL_STACK];
-    float stack_t[TRAVERSAL_STACK];
-    int sp = 0;
-    const bool parallel = P.cam.model == 0;
-    const float spread = parallel ? R : b.lens;
-    uint32_t cur = 0, visits = 0;
-    float cur_t = 0.0f;
-    while (true) {
-        if (cur >= n_nodes4) {
-            L.complete = 0.0f;
-            break;
-        }
-        if (++visits > LIST_VISITS || L.complete < INF) {  // what is left to visit begins here
-            L.complete = fminf(L.complete, cur_t * back);
-            while (sp > 0)
-                L.complete = fminf(L.complete, stack_t[--sp] * back);
-            break;
-        }
-        const float4* np = nodes4 + 8 * size_t(cur);
-        const float4 lx = ldg4(np), hx = ldg4(np + 1), ly = ldg4(np + 2), hy = ldg4(np + 3),
-                     lz = ldg4(np + 4), hz = ldg4(np + 5);
-        const uint4 ci = __ldg(reinterpret_cast<const uint4*>(np + 6));
-        const uint4 cc = __ldg(reinterpret_cast<const uint4*>(np + 7));
-        uint32_t key[4];
-        auto child = [&](float x0, float x1, float y0, float y1, float z0, float z1,
-                         uint32_t first, uint32_t count, uint32_t k) {
-            float te;
-            if (count == EMPTY_CHILD ||
-                !slab(ray, make_float4(x0 - R, y0 - R, z0 - R, 0.0f),
-                      make_float4(x1 + R, y1 + R, z1 + R, 0.0f), INF, te) ||
-                te * back > L.reach())
-                return 0xFFFFFFFFu;
-            if (count == 0u)
-                return (__float_as_uint(te) & ~3u) | k;
-            if (first > n_prims || count > n_prims - first) {
-                L.complete = 0.0f;
-                return 0xFFFFFFFFu;
-            }
-            for (uint32_t s = first; s < first + count; ++s) {
-                const float4 q = ldg4(combined ? sc.leaf_data + 2 * size_t(s) : g.leaf_data + s);
-                const V3 c = v3(q.x, q.y, q.z);
-                const SphereBounds sb = sphere_bounds(b, parallel, spread, c, q.w,
-                                                      [&](float tau) { return b.at(tau); });
-                const float a2 = axis_dist2(b, c);
-                if (a2 <= sb.inner2)
-                    L.certain = fminf(L.certain, sb.t_hi);
-                if (a2 <= sb.reach * sb.reach)
-                    L.add(s, sb.t_lo);
-            }
-            return 0xFFFFFFFFu;
-        };
-        key[0] = child(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, ci.x, cc.x, 0);
-        key[1] = child(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, ci.y, cc.y, 1);
-        key[2] = child(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, ci.z, cc.z, 2);
-        key[3] = child(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, ci.w, cc.w, 3);
-        cswap(key[0], key[1]);
-        cswap(key[2], key[3]);
-        cswap(key[0], key[2]);
-        cswap(key[1], key[3]);
-        cswap(key[1], key[2]);
-#pragma unroll
-        for (int k = 3; k >= 0; --k) {
-            if (key[k] == 0xFFFFFFFFu)
-                continue;
-            if (sp < TRAVERSAL_STACK) {
-                stack_node[sp] = pick4(ci.x, ci.y, ci.z, ci.w, key[k] & 3u);
-                stack_t[sp] = __uint_as_float(key[k] & ~3u);
-                ++sp;
-            } else {
-                L.complete = 0.0f;
-            }
-        }
-        bool found = false;
-        while (sp > 0) {
-            --sp;
-            if (stack_t[sp] * back <= L.reach()) {
-                cur = stack_node[sp];
-                cur_t = stack_t[sp];
-                found = true;
-                break;
-            }
-        }
-        if (!found)
-            break;
-    }
-    L.store(to);
-}
-
 }  // namespace
 
 // Camera rays per pixel, and in all, from which building the lists pays (16 samples of a 200k-sphere
@@ -644,9 +501,7 @@ constexpr double LIST_WIDEST = 0.6;
 
 bool lists_possible(const FrameParams& P)
 {
-    return P.scene.grid.n_cells != 0 ||
-           (P.bvh_width == 4 && (P.type_mask & ~MASK_SPHERES) == 0u && P.type_mask != 0u &&
-            P.refill_geom != -1);
+    return P.scene.grid.n_cells != 0;
 }
 
 bool lists_pay(const FrameParams& P, uint32_t samples)
@@ -654,8 +509,6 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
     if (samples < LIST_MIN_SAMPLES || uint64_t(P.w) * P.h * samples < LIST_MIN_RAYS)
         return false;
     const GridDev& G = P.scene.grid;
-    if (G.n_cells == 0)
-        return true;
     if (G.nx <= 1 || G.ny <= 1 || G.nz <= 1)
         return false;  // a camera ray crosses only a cell or two of a flat layer
     // the beam's radius in the middle of the grid: one pixel, and the lens away from the focus
@@ -683,9 +536,7 @@ void launch_pixel_lists(const FrameParams& P, uint2* lists, cudaStream_t st)
 {
     const uint32_t tiles = ((P.w + 7u) >> 3) * ((P.h + 3u) >> 2);
     const uint32_t blocks = (tiles + 3u) / 4u;
-    if (P.scene.grid.n_cells == 0)
-        k_pixel_lists_bvh<<<blocks, 128, 0, st>>>(P, lists);
-    else if (P.scene.grid.parts)
+    if (P.scene.grid.parts)
         k_pixel_lists_grid<true><<<blocks, 128, 0, st>>>(P, lists);
     else
         k_pixel_lists_grid<false><<<blocks, 128, 0, st>>>(P, lists);

@@ -973,8 +973,6 @@ void launch_path_primary_shade(const FrameParams& P, const PathState& S, bool re
                        : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, true>
                                  : k_path_primary_shade<4, MASK_GRID_PARTS_NO_MESH, true>)
                     : FR_GRID_KERNEL(k_path_primary_shade, gk);
-    else if (P.lists)
-        k = k_path_primary_shade<4, MASK_SPHERES, true>;
     k<<<(n_items + 255) / 256, 256, 0, st>>>(P, S);
 }
 
@@ -1091,12 +1089,10 @@ void launch_preview(const FrameParams& P, uint32_t aa_n, uint2* hits, cudaStream
                                  : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 16>);
         if (P.lists) {
             const int gk = grid_kind(P);
-            k = g32 ? (gk == 0   ? k_preview_warp<4, MASK_SPHERES, 32, true>
-                       : gk == 1 ? k_preview_warp<4, MASK_GRID, 32, true>
+            k = g32 ? (gk == 1   ? k_preview_warp<4, MASK_GRID, 32, true>
                        : gk == 2 ? k_preview_warp<4, MASK_GRID_PARTS, 32, true>
                                  : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 32, true>)
-                    : (gk == 0   ? k_preview_warp<4, MASK_SPHERES, 16, true>
-                       : gk == 1 ? k_preview_warp<4, MASK_GRID, 16, true>
+                    : (gk == 1   ? k_preview_warp<4, MASK_GRID, 16, true>
                        : gk == 2 ? k_preview_warp<4, MASK_GRID_PARTS, 16, true>
                                  : k_preview_warp<4, MASK_GRID_PARTS_NO_MESH, 16, true>);
         }

@@ -205,9 +205,9 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *   "pixel_lists"   camera rays take their closest hits from per-pixel lists of the primitives
  *                   the pixel's beam can meet, built once per render, where the lists answer
  *                   them: 0: never (every ray walks the acceleration structure); 1: for every
- *                   scene traced through a grid or a tree over spheres; 2 (default): where
- *                   they are expected to pay (at least 16 samples per pixel, 3 million camera
- *                   rays, beams thinner than the primitives).  The same images in every case.
+ *                   scene traced through a grid; 2 (default): where they are expected to pay
+ *                   (at least 16 samples per pixel, 3 million camera rays, beams thinner than
+ *                   the primitives).  The same images in every case.
  *   "wave"          1 (default): bounces of scenes traced through a sphere grid trace and shade in
  *                   separate passes over queues of whole path records (at least 2M path
  *                   slots), the tracing with per-lane refill; 0: fused bounces as below.  The
