@@ -89,6 +89,9 @@ struct GridDev {
     const uint32_t* cell_start;
     const float4* ref_sphere;
     const uint32_t* ref_prim;
+    // parts: per reference a sphere (x, y, z, r): a sphere reference's own, else one around the
+    // primitive with r negative (-inf: none known)
+    const float4* ref_bound;
     // 1: a grid over the primitives of several geometries (or one non-sphere geometry); its
     // references are records laid out as a combined tree's leaf slots (SceneDev::leaf_data,
     // leaf_geom, order), and ref_sphere / ref_prim / geom are unused

@@ -486,6 +486,36 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
         L.store(out + size_t(LIST_WORDS) * (size_t(j) * P.w + i));
 }
 
+__global__ void __launch_bounds__(256) k_part_bounds(SceneDev sc, uint32_t n, float4* bound)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n)
+        return;
+    const uint32_t gw = __ldg(sc.leaf_geom + s);
+    const PartShape p = part_shape(sc, s, gw);
+    if (p.sphere) {
+        bound[s] = make_float4(p.c.x, p.c.y, p.c.z, p.e.x);
+        return;
+    }
+    float r;
+    if (int(gw >> PART_TYPE_SHIFT) == FR_GEOM_CYLINDER) {
+        const float4 a = ldg4(sc.leaf_data + 2 * size_t(s)), b = ldg4(sc.leaf_data + 2 * size_t(s) + 1);
+        const V3 h = v3(b.x - a.x, b.y - a.y, b.z - a.z);
+        r = 0.5f * root(dot(h, h)) + fabsf(a.w);
+    } else {
+        r = p.e.x;  // a bounding radius about the position
+        // The polyhedron test stops, and accepts, once the entry and the exit found so far are
+        // equal, without looking at the planes left: a ray that crosses the extension of an edge
+        // can be hit outside the polyhedron, though (as the test's own box test asks) only if it
+        // meets the box of that radius.
+        if (int(gw >> PART_TYPE_SHIFT) == FR_GEOM_POLYHEDRON)
+            r *= 1.7320509f;
+    }
+    const float scale = fmaxf(fmaxf(fabsf(p.c.x), fabsf(p.c.y)), fabsf(p.c.z)) + r;
+    r = r * (1.0f + 1e-5f) + 2e-4f * scale + 2e-5f;
+    bound[s] = make_float4(p.c.x, p.c.y, p.c.z, p.regular && r < INF ? -r : -INF);
+}
+
 }  // namespace
 
 // Camera rays per pixel, and in all, from which building the lists pays (16 samples of a 200k-sphere
@@ -525,6 +555,12 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
         rho = rho * s + 0.5 * std::fabs(double(k.aperture)) * std::max(std::fabs(1.0 - s), half);
     }
     return rho <= LIST_WIDEST * G.mean_radius;
+}
+
+void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStream_t st)
+{
+    if (n)
+        k_part_bounds<<<(n + 255) / 256, 256, 0, st>>>(sc, n, bound);
 }
 
 size_t pixel_list_words(const FrameParams& P)

@@ -965,9 +965,13 @@ void launch_path_primary_shade(const FrameParams& P, const PathState& S, bool re
     auto k = pick(P, k_path_primary_shade<2, MASK_SPHERES>, k_path_primary_shade<2, MASK_ALL>,
                   k_path_primary_shade<4, MASK_SPHERES>, k_path_primary_shade<4, MASK_ALL>);
     const int gk = grid_kind(P);
-    if (rec && gk == 1)
-        k = P.lists ? k_path_primary_shade<4, MASK_GRID, true, true>
-                    : k_path_primary_shade<4, MASK_GRID, false, true>;
+    if (rec && gk)
+        k = P.lists ? (gk == 1   ? k_path_primary_shade<4, MASK_GRID, true, true>
+                       : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, true, true>
+                                 : k_path_primary_shade<4, MASK_GRID_PARTS_NO_MESH, true, true>)
+                    : (gk == 1   ? k_path_primary_shade<4, MASK_GRID, false, true>
+                       : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, false, true>
+                                 : k_path_primary_shade<4, MASK_GRID_PARTS_NO_MESH, false, true>);
     else if (gk)
         k = P.lists ? (gk == 1   ? k_path_primary_shade<4, MASK_GRID, true>
                        : gk == 2 ? k_path_primary_shade<4, MASK_GRID_PARTS, true>

@@ -65,7 +65,7 @@ struct PathState {
 
 struct LaunchShape {
     int trace_grid[3];       // packed queues: trace, shade and tail kernels, per grid kind
-    int shade_rec_grid[3];   // [sphere grid|parts grid|parts grid without meshes]
+    int shade_rec_grid;      // [sphere grid|parts grid|parts grid without meshes]
     int tail_rec_grid[3];
     int shade_grid;
     int shade_grid_occ[2];   // shade kernel compiled for 3|4 blocks per SM
@@ -104,6 +104,8 @@ void launch_path_bounce(const FrameParams& P, const PathState& S, int iteration,
 // The remaining bounces of every path in queue (iteration & 1) in one launch (k_path_tail).
 void launch_path_tail(const FrameParams& P, const PathState& S, int iteration,
                       const LaunchShape& shape, cudaStream_t st);
+// The spheres around the references of a grid over parts (GridDev::ref_bound), n references.
+void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStream_t st);
 // Per-pixel primitive lists of the frame's camera rays (beam.cuh: LIST_WORDS uint2 per pixel,
 // row by row), for scenes where lists are possible; lists_pay: `samples` camera rays per pixel are
 // expected to gain more than the lists cost.

@@ -15,6 +15,7 @@
 // of a 200k-sphere frame moves 334 MB instead of 914 MB through HBM (0.17 against 0.28 ms).
 // Against the fused bounce and tail kernels: 1M spheres 1080p, 256 samples 54.4 -> 44.4 ms a frame;
 // 1000 spheres with 32 light samples 50.8 -> 34.5 ms; 200k spheres, 16 samples 2.87 -> 2.72 ms.
+// The mixed scene of 280k primitives, 1280x720, 128 samples: 51.4 -> 31.3 ms.
 // What bounds k_wave_trace now: issue (72%), with 15 of 32 lanes active on average (a lane's
 // iteration takes the test, the square root or the step, and not all need each).
 #include "path_device.cuh"
@@ -26,13 +27,12 @@ namespace {
 // Idle lanes of a warp before they take new rays (one atomic per refill).
 constexpr uint32_t WAVE_REFILL = 8;
 
-// Walk of one ray through a sphere grid, one iteration at a time.  Each axis keeps the plane the
-// ray leaves the current cell through as a whole number of cells (p), so that the distance to it is
+// Walk of one ray through a grid, one iteration at a time.  Each axis keeps the plane the ray
+// leaves the current cell through as a whole number of cells (p), so that the distance to it is
 // recomputed from the plane's position at every step, exactly as grid_walk_visit does.
-struct SphereWalk {
+struct CellWalk {
     RayK ray;
-    float tmax;
-    uint32_t slot;       // reference of the closest hit so far
+    float tmax;          // distance of the closest hit so far
     float px, py, pz;    // exit planes of the cell last stepped to (the one after the current)
     float tx, ty, tz;    // distances to them
     float t_out;         // distance at which the ray leaves the grid
@@ -73,11 +73,10 @@ struct SphereWalk {
         tz = fmaf(fmaf(pz, G.hz, G.loz), ray.inv.z, ray.oinv.z);
     }
     // false: the ray misses the grid
-    __device__ __forceinline__ bool begin(const GridDev& G, V3 o, V3 d, TraceCount& tc)
+    __device__ __forceinline__ bool begin_cells(const GridDev& G, V3 o, V3 d, TraceCount& tc)
     {
         ray = make_rayk(o, d);
         tmax = __int_as_float(0x7f800000);
-        slot = MISS;
         GridWalk W;
         if (!grid_walk_begin(G, ray, W))
             return false;
@@ -96,9 +95,58 @@ struct SphereWalk {
         tc.prim += end - k;
         return true;
     }
-    // one iteration; false once the walk is over
-    __device__ __forceinline__ bool step(const GridDev& G, float tnear, TraceCount& tc)
+    // the next cell, once every reference of the current one is tested; false when the walk is over
+    __device__ __forceinline__ bool next_cell(const GridDev& G, TraceCount& tc)
     {
+        if (tmax <= t_cell || !more)
+            return false;
+        k = nk;
+        end = nend;
+        look_ahead(G);
+        tc.box += 1;
+        tc.prim += end - k;
+        return true;
+    }
+};
+
+// The line distance test of sphere_t for the spheres (c, r) of two references, up to its square
+// root: most lines miss, and of the spheres they meet half lie behind (b < 0 and |b| above the
+// root by more than its rounding, so that both distances are negative).
+struct LineTest {
+    float b, d;  // projection of the centre, discriminant
+    bool c;      // the sphere may be hit
+    __device__ __forceinline__ LineTest(const RayK& ray, V3 centre, float r)
+    {
+        const V3 v = centre - ray.o;
+        b = dot(v, ray.d);
+        const float s = b * b;
+        d = s - dot(v, v) + r * r;
+        c = !(d < 0) && !(b < 0.0f && d < 0.999998f * s);
+    }
+    // sphere_t's distance; false when it has none
+    __device__ __forceinline__ static bool distance(float b, float d, float& t)
+    {
+        const float root = sqrtf(d);
+        t = b - root;
+        if (!(t > SPHERE_EPS))
+            t = b + root;
+        return t > SPHERE_EPS;
+    }
+};
+
+struct SphereWalk : CellWalk {
+    static constexpr bool DEFERS = false;
+    uint32_t slot;  // reference of the closest hit so far
+
+    __device__ __forceinline__ bool begin(const FrameParams& P, V3 o, V3 d, TraceCount& tc)
+    {
+        slot = MISS;
+        return begin_cells(P.scene.grid, o, d, tc);
+    }
+    // one iteration; false once the walk is over
+    __device__ __forceinline__ bool step(const FrameParams& P, float tnear, TraceCount& tc)
+    {
+        const GridDev& G = P.scene.grid;
         // exact tie with the closest hit so far: the lower sphere index wins (one geometry)
         const auto tie = [&](uint32_t r) {
             return slot != MISS && __ldg(G.ref_prim + r) < __ldg(G.ref_prim + slot);
@@ -107,52 +155,129 @@ struct SphereWalk {
             const bool two = k + 1u < end;
             const float4 q0 = ldg4(G.ref_sphere + k);
             const float4 q1 = ldg4(G.ref_sphere + (two ? k + 1u : k));
-            // sphere_t of both, up to its square root: most lines miss, and of the spheres they
-            // meet half lie behind (b < 0 and |b| above the root by more than its rounding, so
-            // that both distances are negative); the rest is one section for either sphere, which
-            // a warp enters once per iteration (a second time where a lane needs both)
-            const V3 v0 = v3(q0.x, q0.y, q0.z) - ray.o, v1 = v3(q1.x, q1.y, q1.z) - ray.o;
-            const float b0 = dot(v0, ray.d), b1 = dot(v1, ray.d);
-            const float s0 = b0 * b0, s1 = b1 * b1;
-            const float d0 = s0 - dot(v0, v0) + q0.w * q0.w, d1 = s1 - dot(v1, v1) + q1.w * q1.w;
-            bool c0 = !(d0 < 0) && !(b0 < 0.0f && d0 < 0.999998f * s0);
-            bool c1 = two && !(d1 < 0) && !(b1 < 0.0f && d1 < 0.999998f * s1);
-            while (c0 || c1) {
-                const float b = c0 ? b0 : b1, root = sqrtf(c0 ? d0 : d1);
-                const uint32_t r = c0 ? k : k + 1u;
-                if (c0)
-                    c0 = false;
+            LineTest l0(ray, v3(q0.x, q0.y, q0.z), q0.w), l1(ray, v3(q1.x, q1.y, q1.z), q1.w);
+            l1.c = l1.c && two;
+            // one section for either sphere, which a warp enters once per iteration (a second
+            // time where a lane needs both)
+            while (l0.c || l1.c) {
+                float t;
+                const bool hit = LineTest::distance(l0.c ? l0.b : l1.b, l0.c ? l0.d : l1.d, t);
+                const uint32_t r = l0.c ? k : k + 1u;
+                if (l0.c)
+                    l0.c = false;
                 else
-                    c1 = false;
-                float t = b - root;
-                if (!(t > SPHERE_EPS))
-                    t = b + root;
-                if (t > SPHERE_EPS && tnear < t && (t < tmax || (t == tmax && tie(r)))) {
+                    l1.c = false;
+                if (hit && tnear < t && (t < tmax || (t == tmax && tie(r)))) {
                     tmax = t;
                     slot = r;
                 }
             }
             k += 2u;
         }
-        if (k >= end) {
-            if (tmax <= t_cell || !more)
-                return false;
-            k = nk;
-            end = nend;
-            look_ahead(G);
-            tc.box += 1;
-            tc.prim += end - k;
-        }
-        return true;
+        return k < end || next_cell(G, tc);
     }
-    __device__ __forceinline__ uint2 hit(const GridDev& G) const
+    __device__ __forceinline__ uint2 hit(const FrameParams& P) const
     {
+        const GridDev& G = P.scene.grid;
         return slot == MISS ? make_uint2(MISS, 0u) : make_uint2(G.geom, __ldg(G.ref_prim + slot));
     }
 };
 
+// Walk through a grid over parts.  Every reference is first tested by a sphere (GridDev::ref_bound:
+// the sphere itself, or one around the primitive, its radius negative), two references per
+// iteration as above; a primitive of another type whose sphere the ray meets waits (pend) until
+// enough lanes of the warp hold one, and then its own test, with its own box test before it,
+// runs for all of them together (parts_cell_test).
+template <uint32_t TYPES>
+struct PartsWalk : CellWalk {
+    static constexpr bool DEFERS = true;
+    uint32_t hg, hp;          // closest hit so far
+    uint32_t last_g, last_p;  // see parts_cell_test
+    uint32_t pend;            // reference whose test waits (MISS: none)
+
+    __device__ __forceinline__ bool begin(const FrameParams& P, V3 o, V3 d, TraceCount& tc)
+    {
+        hg = last_g = pend = MISS;
+        hp = last_p = 0;
+        return begin_cells(P.scene.grid, o, d, tc);
+    }
+    // Sphere test of reference r: true for a primitive of another type to test.
+    __device__ __forceinline__ LineTest line(const FrameParams& P, uint32_t r, float& radius) const
+    {
+        const float4 q = ldg4(P.scene.grid.ref_bound + r);
+        const V3 c = v3(q.x, q.y, q.z);
+        radius = q.w;
+        if (q.w < 0.0f) {
+            // widened by what the primitive's own test may be off by (see SPHERE_SLACK: a cylinder's
+            // discriminant is off by up to 1.25e-6 of the squared distance)
+            const V3 v = c - ray.o;
+            const float far = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z));
+            radius = fmaf(far, 2.2e-3f, -q.w);
+        }
+        LineTest l(ray, c, radius);
+        if (q.w < 0.0f) {
+            if (l.b - radius > tmax)
+                l.c = false;  // wholly beyond the closest hit
+            radius = -1.0f;
+        }
+        return l;
+    }
+    __device__ __forceinline__ bool step(const FrameParams& P, float tnear, TraceCount& tc)
+    {
+        const SceneDev& sc = P.scene;
+        if (k < end) {
+            const bool two = k + 1u < end;
+            float r0, r1;
+            LineTest l0 = line(P, k, r0), l1 = line(P, two ? k + 1u : k, r1);
+            l1.c = l1.c && two;
+            while (l0.c || l1.c) {
+                const bool first = l0.c;
+                const uint32_t r = first ? k : k + 1u;
+                if ((first ? r0 : r1) < 0.0f) {
+                    pend = r;
+                    k = r + 1u;  // the references after it wait with it
+                    return true;
+                }
+                float t;
+                const bool hit = LineTest::distance(first ? l0.b : l1.b, first ? l0.d : l1.d, t);
+                if (first)
+                    l0.c = false;
+                else
+                    l1.c = false;
+                if (hit && tnear < t && t <= tmax) {
+                    const uint32_t g = __ldg(sc.leaf_geom + r) & ((1u << PART_TYPE_SHIFT) - 1u);
+                    const uint32_t p = __ldg(sc.order + r);
+                    if (t < tmax || tie_wins(g, hg, [&]() { return p; }, [&]() { return hp; })) {
+                        tmax = t;
+                        hg = g;
+                        hp = p;
+                    }
+                }
+            }
+            k += 2u;
+        }
+        return k < end || next_cell(sc.grid, tc);
+    }
+    // the waiting primitive's own test
+    __device__ __forceinline__ void resolve(const FrameParams& P, float tnear)
+    {
+        TraceCount none;  // counted with its cell
+        parts_cell_test<TYPES>(P.scene, ray, pend, pend + 1u, tnear, tmax, hg, hp, last_g, last_p,
+                               none);
+        pend = MISS;
+    }
+    __device__ __forceinline__ uint2 hit(const FrameParams&) const
+    {
+        return make_uint2(hg, hg == MISS ? 0u : hp);
+    }
+};
+
+// Lanes of a warp with a waiting primitive before their tests run.
+constexpr uint32_t WAVE_PENDING = 8;  // (the primitives' own tests ran with some 2 lanes of a warp
+                                     // in the fused kernels' walk)
+
 template <class Walk>
-__global__ void __launch_bounds__(256, 4) k_wave_trace(FrameParams P, PathState S, int q)
+__global__ void __launch_bounds__(256, Walk::DEFERS ? 3 : 4) k_wave_trace(FrameParams P, PathState S, int q)
 {
     const uint32_t count = S.ctr[q];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -161,7 +286,6 @@ __global__ void __launch_bounds__(256, 4) k_wave_trace(FrameParams P, PathState 
     }
     const float4* rec_o = S.rec_o[q];
     const float4* rec_d = S.rec_d[q];
-    const GridDev& G = P.scene.grid;
     const uint32_t lane = lane_id();
     const uint32_t below = (1u << lane) - 1u;
     TraceCount tc;
@@ -180,7 +304,7 @@ __global__ void __launch_bounds__(256, 4) k_wave_trace(FrameParams P, PathState 
             if (!active) {
                 i = base + uint32_t(__popc(idle & below));
                 if (i < count) {
-                    active = W.begin(G, xyz(ld_cs(rec_o + i)), xyz(ld_cs(rec_d + i)), tc);
+                    active = W.begin(P, xyz(ld_cs(rec_o + i)), xyz(ld_cs(rec_d + i)), tc);
                     if (!active)
                         st_cs(S.hit + i, make_uint2(MISS, 0u));
                 }
@@ -190,10 +314,19 @@ __global__ void __launch_bounds__(256, 4) k_wave_trace(FrameParams P, PathState 
         }
 #pragma unroll 1
         for (int r = 0; r < 3; ++r) {
-            if (active && !W.step(G, PATH_TNEAR, tc)) {
-                st_cs(S.hit + i, W.hit(G));
+            bool walks = active;
+            if constexpr (Walk::DEFERS)
+                walks = active && W.pend == MISS;
+            if (walks && !W.step(P, PATH_TNEAR, tc)) {
+                st_cs(S.hit + i, W.hit(P));
                 active = false;
             }
+        }
+        if constexpr (Walk::DEFERS) {
+            const bool waits = active && W.pend != MISS;
+            const uint32_t n = uint32_t(__popc(__ballot_sync(0xffffffffu, waits)));
+            if (n && (n >= WAVE_PENDING || !__any_sync(0xffffffffu, active && !waits)) && waits)
+                W.resolve(P, PATH_TNEAR);
         }
     }
     flush_counts(tc, P.stats + 3);
@@ -334,6 +467,8 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_wave_tail(FramePara
     flush_counts(tc, P.stats + 3);
 }
 
+constexpr uint32_t NO_MESH = MASK_GRID_PARTS_NO_MESH & MASK_ALL;
+
 template <class K> int fill(K kernel, int num_sms)
 {
     int n = 0;
@@ -345,29 +480,45 @@ template <class K> int fill(K kernel, int num_sms)
 
 void wave_launch_shape(int num_sms, LaunchShape& s)
 {
-    for (int k = 0; k < 3; ++k) {
-        s.trace_grid[k] = fill(k_wave_trace<SphereWalk>, num_sms);
-        s.shade_rec_grid[k] = fill(k_wave_shade, num_sms);
-        s.tail_rec_grid[k] = fill(k_wave_tail<MASK_GRID>, num_sms);
-    }
+    s.trace_grid[0] = fill(k_wave_trace<SphereWalk>, num_sms);
+    s.trace_grid[1] = fill(k_wave_trace<PartsWalk<MASK_ALL>>, num_sms);
+    s.trace_grid[2] = fill(k_wave_trace<PartsWalk<NO_MESH>>, num_sms);
+    s.shade_rec_grid = fill(k_wave_shade, num_sms);
+    s.tail_rec_grid[0] = fill(k_wave_tail<MASK_GRID>, num_sms);
+    s.tail_rec_grid[1] = fill(k_wave_tail<MASK_GRID_PARTS>, num_sms);
+    s.tail_rec_grid[2] = fill(k_wave_tail<MASK_GRID_PARTS_NO_MESH>, num_sms);
+}
+
+// 0: a sphere grid, 1: a grid over parts, 2: one without meshes.
+static int wave_kind(const FrameParams& P)
+{
+    return !P.scene.grid.parts ? 0 : (P.type_mask & (1u << FR_GEOM_MESH)) ? 1 : 2;
 }
 
 void launch_wave_trace(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
                        cudaStream_t st)
 {
-    k_wave_trace<SphereWalk><<<shape.trace_grid[0], 256, 0, st>>>(P, S, q);
+    const int gk = wave_kind(P);
+    auto k = gk == 0   ? k_wave_trace<SphereWalk>
+             : gk == 1 ? k_wave_trace<PartsWalk<MASK_ALL>>
+                       : k_wave_trace<PartsWalk<NO_MESH>>;
+    k<<<shape.trace_grid[gk], 256, 0, st>>>(P, S, q);
 }
 
 void launch_wave_shade(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
                        cudaStream_t st)
 {
-    k_wave_shade<<<shape.shade_rec_grid[0], 256, 0, st>>>(P, S, q);
+    k_wave_shade<<<shape.shade_rec_grid, 256, 0, st>>>(P, S, q);
 }
 
 void launch_wave_tail(const FrameParams& P, const PathState& S, int q, const LaunchShape& shape,
                       cudaStream_t st)
 {
-    k_wave_tail<MASK_GRID><<<shape.tail_rec_grid[0], 256, 0, st>>>(P, S, q);
+    const int gk = wave_kind(P);
+    auto k = gk == 0   ? k_wave_tail<MASK_GRID>
+             : gk == 1 ? k_wave_tail<MASK_GRID_PARTS>
+                       : k_wave_tail<MASK_GRID_PARTS_NO_MESH>;
+    k<<<shape.tail_rec_grid[gk], 256, 0, st>>>(P, S, q);
 }
 
 }  // namespace fr

@@ -208,7 +208,7 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   scene traced through a grid; 2 (default): where they are expected to pay
  *                   (at least 16 samples per pixel, 3 million camera rays, beams thinner than
  *                   the primitives).  The same images in every case.
- *   "wave"          1 (default): bounces of scenes traced through a sphere grid trace and shade in
+ *   "wave"          1 (default): bounces of scenes traced through a grid trace and shade in
  *                   separate passes over queues of whole path records (at least 2M path
  *                   slots), the tracing with per-lane refill; 0: fused bounces as below.  The
  *                   same images in both cases.

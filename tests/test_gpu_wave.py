@@ -4,7 +4,8 @@ Both follow the same paths with the same arithmetic, so images and ray counts mu
 for bit: wavefronts long enough for several trace-and-shade passes and ones the tail kernel takes
 after the first, one and several light samples per camera ray (the second packed queue then lies
 in arrays of its own, and a lane restarts light samples), image sizes that are no multiple of a
-tile, a single sphere, and rays that leave the scene at once.
+tile, a single sphere, and rays that leave the scene at once; spheres, and grids over parts with
+every type of primitive, whose own tests wait for one another there.
 """
 
 import numpy
@@ -30,7 +31,38 @@ def _scene(dev, n, box, radius, at, outline=0.0):
     return scene
 
 
+def _mixed(dev, scale=0.01):
+    from fresnel_b200 import workloads
+    return workloads.config3(dev, scale=scale)
+
+
+def _layers(dev):
+    from fresnel_b200 import workloads
+    return workloads.polygons(dev, nx=20, ny=16, spheres=300)
+
+
+def _odd_cubes(dev):
+    """Cubes whose stated bounding radius is too small, some of them scaled by their quaternions."""
+    import fresnel_b200 as fresnel
+    from fresnel_b200 import workloads
+    rng = numpy.random.default_rng(8)
+    scene = fresnel.Scene(dev, lights=fresnel.light.rembrandt())
+    info = workloads.unit_cube_planes()
+    info["radius"] = 0.6
+    pos = rng.uniform(-5, 5, (700, 3)).astype(numpy.float32)
+    q = workloads.random_quaternions(rng, 700)
+    q[::3] *= 0.8
+    fresnel.geometry.ConvexPolyhedron(scene, info, position=pos, orientation=q,
+                                      color=(0.7, 0.4, 0.2), outline_width=0.02)
+    scene.camera = fresnel.camera.Orthographic.fit(scene)
+    return scene
+
+
 CASES = {  # scene, image size, samples, light samples
+    "mixed": (_mixed, (160, 130), 250, 1),
+    "mixed_lights": (_mixed, (161, 97), 150, 2),
+    "layers": (_layers, (160, 128), 220, 1),
+    "odd_cubes": (_odd_cubes, (130, 130), 200, 1),
     "dense": (dict(n=6000, box=20.0, radius=0.6, at=(20.0, 12.0, 26.0)), (161, 129), 250, 1),
     "dense_lights": (dict(n=6000, box=20.0, radius=0.6, at=(20.0, 12.0, 26.0), outline=0.05),
                      (161, 129), 120, 3),
@@ -45,7 +77,7 @@ def test_packed_queues_give_the_fused_kernels_images(gpu_device, name):
     import fresnel_b200 as fresnel
     args, size, samples, lights = CASES[name]
     option = gpu_device._device.setOption
-    scene = _scene(gpu_device, **args)
+    scene = args(gpu_device) if callable(args) else _scene(gpu_device, **args)
     out = []
     try:
         for wave in (0, 1):
