@@ -1063,11 +1063,12 @@ void prepare_lists(fr_device* dev, FrameParams& P, uint32_t samples)
 
 fr_status check_status(fr_device* dev)
 {
-    uint32_t st = 0;
-    FR_CUDA(cudaMemcpyAsync(&st, dev->status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                            dev->stream),
+    // into a page-locked word: a copy to the stack is staged by the driver
+    FR_CUDA(cudaMemcpyAsync(dev->h_count + 3, dev->status.ptr, sizeof(uint32_t),
+                            cudaMemcpyDeviceToHost, dev->stream),
             "reading the device status");
     FR_CUDA(cudaStreamSynchronize(dev->stream), "render");
+    const uint32_t st = dev->h_count[3];
     if (st) {
         FR_CUDA(cudaMemsetAsync(dev->status.ptr, 0, sizeof(uint32_t), dev->stream), "status reset");
         return fail(FR_ERR_DEVICE_LIMIT,
@@ -1886,8 +1887,7 @@ fr_status fr_tracer_clear(fr_tracer* t)
     size_t n = size_t(t->w) * t->h;
     FR_CUDA(cudaMemsetAsync(t->linear.ptr, 0, n * sizeof(float4), t->dev->stream), "clear");
     FR_CUDA(cudaMemsetAsync(t->srgb.ptr, 0, n * sizeof(uint32_t), t->dev->stream), "clear");
-    FR_CUDA(cudaStreamSynchronize(t->dev->stream), "clear");
-    return FR_OK;
+    return FR_OK;  // whatever reads or writes the outputs next is on the same stream
 }
 
 fr_status fr_tracer_render_path(fr_tracer* t, fr_scene* sc, const fr_render_params* p,

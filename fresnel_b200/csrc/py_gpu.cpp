@@ -890,6 +890,14 @@ template <class A> void export_array(py::module_& m, const char* name)
         .def("unmap", &A::unmap)
         .def("unmapRead", &A::unmap_read)
         .def("readCopy", &A::read_copy)
+        // (shape, dtype) without a map(), which downloads a tracer output
+        .def("layout",
+             [](const A& a) {
+                 py::tuple shape(a.shape.size());
+                 for (size_t k = 0; k < a.shape.size(); ++k)
+                     shape[k] = py::int_(a.shape[k]);
+                 return py::make_tuple(shape, py::dtype(a.format));
+             })
         .def_static("streamCopy", &stream_copy);
 }
 

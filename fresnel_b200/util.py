@@ -76,6 +76,12 @@ class Array:
     def __init__(self, buf, geom):
         self.buf = buf
         self.geom = geom
+        layout = getattr(buf, "layout", None)
+        if layout is not None:
+            # mapping a tracer output downloads it, and programs hold many such views: `sample`
+            # and `render` return one, and each use of the output property makes another
+            self.shape, self.dtype = layout()
+            return
         self.buf.map()
         a = numpy.asarray(self.buf)
         self.shape = a.shape
