@@ -218,6 +218,7 @@ struct fr_geometry {
     float outline_width = 0.0f;
     DevArray<float> position, radius, color, points, orientation, vertices, planes;
     DevArray<float> angle;         // polygon: [n] radians; orientation holds their quaternions
+    DevArray<float4> planes4;      // polyhedron: per plane (normal, -normal . origin), (origin, 0)
     DevArray<float4> face_box;     // mesh: per face its local box (lo, hi), padded
     float rounding_radius = 0.0f;  // polygon
     BvhBuffers bvh;
@@ -868,6 +869,7 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
             d.orientation = g->orientation.ptr;
             d.vertices = g->vertices.ptr;
             d.planes = g->planes.ptr;
+            d.planes4 = g->planes4.ptr;
             d.n_faces = g->n_faces;
             d.n_planes = g->n_planes;
             d.n_vertices = g->type == FR_GEOM_POLYGON ? g->n_vertices : 0u;
@@ -1516,6 +1518,7 @@ fr_status fr_geometry_create_polyhedron(fr_scene* scene, const float* origins, c
     // [origin, unit normal, colour] per plane; normals scaled by 1/|n|
     // (fresnel/cpu/GeometryConvexPolyhedron.cc:81-91)
     std::vector<float> pl(size_t(n_planes) * 9);
+    std::vector<float4> pl4(size_t(n_planes) * 2);
     for (uint32_t i = 0; i < n_planes; ++i) {
         V3 nn = v3(normals[3 * i], normals[3 * i + 1], normals[3 * i + 2]);
         nn = div_recip(nn, sqrtf(dot(nn, nn)));
@@ -1529,10 +1532,18 @@ fr_status fr_geometry_create_polyhedron(fr_scene* scene, const float* origins, c
         q[6] = colors[3 * i];
         q[7] = colors[3 * i + 1];
         q[8] = colors[3 * i + 2];
+        const V3 p = v3(q[0], q[1], q[2]);
+        pl4[2 * size_t(i)] = make_float4(nn.x, nn.y, nn.z, -dot(nn, p));
+        pl4[2 * size_t(i) + 1] = make_float4(p.x, p.y, p.z, 0.0f);
     }
     cudaError_t e = use_device(scene->dev) == FR_OK ? g->planes.reserve(pl.size()) : cudaErrorUnknown;
     if (e == cudaSuccess)
         e = cudaMemcpy(g->planes.ptr, pl.data(), pl.size() * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = g->planes4.reserve(pl4.size());
+    if (e == cudaSuccess)
+        e = cudaMemcpy(g->planes4.ptr, pl4.data(), pl4.size() * sizeof(float4),
+                       cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         delete g;
         return cuda_fail(e, "uploading polyhedron planes");

@@ -56,6 +56,7 @@ struct GeomDev {
     const float* orientation;
     const float* vertices;
     const float* planes;  // [n_planes][9]: origin, unit normal, colour
+    const float4* planes4;  // per plane (unit normal, -normal . origin), (origin, 0)
     uint32_t n_faces;
     uint32_t n_planes;
     uint32_t n_vertices;    // polygon: vertices [n_vertices][2]
@@ -178,8 +179,7 @@ struct PolyHit {
     bool hit;
     float t;
     int plane;
-    V3 n, p;  // local-frame normal and origin of the hit plane
-    V3 ol, dl;
+    V3 ol, dl;  // the ray in the polyhedron's frame
 };
 
 // Exact ties.  A primitive hit at exactly the distance of the closest hit so far (coincident
@@ -211,37 +211,31 @@ __device__ __forceinline__ PolyHit poly_planes(const GeomDev& g, V3 o, V3 d, V3 
     r.hit = false;
     r.t = 0.0f;
     r.plane = 0;
-    r.n = v3(0, 0, 1);
-    r.p = v3(0, 0, 0);
     float t0 = -3.402823466e+38f, t1 = 3.402823466e+38f;
     V3 dl = rotate(conj(q), d);
     V3 ol = rotate(conj(q), o - pos);
     r.ol = ol;
     r.dl = dl;
-    V3 t0n = v3(0, 0, 0), t0p = v3(0, 0, 0), t1n = v3(0, 0, 0), t1p = v3(0, 0, 0);
     int t0_plane = 0, t1_plane = 0;
     for (uint32_t i = 0; i < g.n_planes && t0 < t1; ++i) {
-        const float* pl = g.planes + 9 * i;
-        V3 p = v3(__ldg(pl), __ldg(pl + 1), __ldg(pl + 2));
-        V3 n = v3(__ldg(pl + 3), __ldg(pl + 4), __ldg(pl + 5));
-        float dd = -dot(n, p);
+        const float4 a = ldg4(g.planes4 + 2 * i);
+        const V3 n = v3(a.x, a.y, a.z);
         float denom = dot(n, dl);
-        float t = -(dd + dot(n, ol)) / denom;
-        if (double(fabsf(denom)) < 1e-5) {
-            if (dot(ol - p, n) > 0)
+        float t = -(a.w + dot(n, ol)) / denom;
+        // the reference's fabs(float) < 1e-5 compares in double: true up to the float 1e-5f
+        // (just below 1e-5)
+        if (fabsf(denom) <= 1e-5f) {
+            const float4 p = ldg4(g.planes4 + 2 * i + 1);
+            if (dot(ol - v3(p.x, p.y, p.z), n) > 0)
                 return r;
         } else if (denom < 0) {
             if (t > t0) {
                 t0 = t;
-                t0n = n;
-                t0p = p;
                 t0_plane = int(i);
             }
         } else {
             if (t < t1) {
                 t1 = t;
-                t1n = n;
-                t1p = p;
                 t1_plane = int(i);
             }
         }
@@ -250,17 +244,11 @@ __device__ __forceinline__ PolyHit poly_planes(const GeomDev& g, V3 o, V3 d, V3 
         return r;
     if ((tnear < t0) & ((t0 < tfar) || (t0 == tfar && tie()))) {
         r.hit = true;
-        r.t = tfar = t0;
-        r.n = t0n;
-        r.p = t0p;
-        r.plane = t0_plane;
-        return r;  // the exit (t1 >= t0) cannot be closer
-    }
-    if ((tnear < t1) & ((t1 < tfar) || (t1 == tfar && tie()))) {
+        r.t = t0;
+        r.plane = t0_plane;  // the exit (t1 >= t0) cannot be closer
+    } else if ((tnear < t1) & ((t1 < tfar) || (t1 == tfar && tie()))) {
         r.hit = true;
-        r.t = tfar = t1;
-        r.n = t1n;
-        r.p = t1p;
+        r.t = t1;
         r.plane = t1_plane;
     }
     return r;
@@ -318,7 +306,7 @@ __device__ __forceinline__ PgHit polygon_hit(const GeomDev& g, V3 o, V3 d, float
     const float dd = -dot(n, p);
     const float denom = dot(n, dl);
     const float t = -(dd + dot(n, ol)) / denom;
-    if (double(fabsf(denom)) < 1e-5)
+    if (fabsf(denom) <= 1e-5f)  // the reference's fabs(float) < 1e-5, compared in double
         return r;
     const V3 rh = ol + t * dl;
     // crossing number and the distance to the nearest edge
@@ -1560,48 +1548,56 @@ __device__ __forceinline__ Surface hit_surface(const GeomDev& g, uint32_t prim, 
         Qt q = loadq(g.orientation, prim);
         PolyHit ph = poly_planes(g, o, d, pos, q, tnear, __int_as_float(0x7f800000));
         s.t = ph.t;
-        s.Ng = rotate(q, ph.n);
+        const float4 hn = ldg4(g.planes4 + 2 * ph.plane), hp = ldg4(g.planes4 + 2 * ph.plane + 1);
+        const V3 phn = ph.hit ? v3(hn.x, hn.y, hn.z) : v3(0, 0, 1);
+        const V3 php = ph.hit ? v3(hp.x, hp.y, hp.z) : v3(0, 0, 0);
+        s.Ng = rotate(q, phn);
         const float* pl = g.planes + 9 * ph.plane;
         s.color = lerp(g.color_by_face, loadc3(g.color, prim),
                        c3(__ldg(pl + 6), __ldg(pl + 7), __ldg(pl + 8)));
-        float min_d = 3.402823466e+38f;
+        // distance of the hit point to the nearest edge, as seen along the ray.  It is not negative
+        // and only compared with the outline's width, so without an outline none is needed.
+        s.d_edge = 3.402823466e+38f;
+        if (g.outline_width <= 0.0f)
+            break;
         V3 r_hit = ph.ol + ph.t * ph.dl;
+        const V3 view = div_recip(-ph.dl, sqrtf(dot(ph.dl, ph.dl)));
+        const float d2 = -dot(phn, php);
+        float min_q = __int_as_float(0x7f800000);  // least squared distance (the root is monotonic)
         for (uint32_t i = 0; i < g.n_planes; ++i) {
-            const float* pi = g.planes + 9 * i;
-            V3 p = v3(__ldg(pi), __ldg(pi + 1), __ldg(pi + 2));
-            V3 n = v3(__ldg(pi + 3), __ldg(pi + 4), __ldg(pi + 5));
-            V3 u = cross(n, ph.n);
-            if (double(fabsf(dot(u, u))) >= 1e-5) {
+            const float4 pn = ldg4(g.planes4 + 2 * i);
+            const V3 n = v3(pn.x, pn.y, pn.z);
+            V3 u = cross(n, phn);
+            if (fabsf(dot(u, u)) > 1e-5f) {  // the reference's >= 1e-5, compared in double
                 int maxc;
                 if (fabsf(u.x) > fabsf(u.y))
                     maxc = (fabsf(u.x) > fabsf(u.z)) ? 1 : 3;
                 else
                     maxc = (fabsf(u.y) > fabsf(u.z)) ? 2 : 3;
                 V3 x0 = v3(0, 0, 0);
-                float d1 = -dot(n, p);
-                float d2 = -dot(ph.n, ph.p);
+                const float d1 = pn.w;
                 if (maxc == 1) {
-                    x0.y = (d2 * n.z - d1 * ph.n.z) / u.x;
-                    x0.z = (d1 * ph.n.y - d2 * n.y) / u.x;
+                    x0.y = (d2 * n.z - d1 * phn.z) / u.x;
+                    x0.z = (d1 * phn.y - d2 * n.y) / u.x;
                 } else if (maxc == 2) {
-                    x0.x = (d1 * ph.n.z - d2 * n.z) / u.y;
-                    x0.z = (d2 * n.x - d1 * ph.n.x) / u.y;
+                    x0.x = (d1 * phn.z - d2 * n.z) / u.y;
+                    x0.z = (d2 * n.x - d1 * phn.x) / u.y;
                 } else {
-                    x0.x = (d2 * n.y - d1 * ph.n.y) / u.z;
-                    x0.y = (d1 * ph.n.x - d2 * n.x) / u.z;
+                    x0.x = (d2 * n.y - d1 * phn.y) / u.z;
+                    x0.y = (d1 * phn.x - d2 * n.x) / u.z;
                 }
-                V3 view = div_recip(-ph.dl, sqrtf(dot(ph.dl, ph.dl)));
                 u = u - dot(u, view) * view;
                 V3 w = x0 - r_hit;
                 V3 w_perp = w - dot(w, view) * view;
                 x0 = r_hit + w_perp;
                 V3 vv = cross(u, x0 - r_hit);
-                float dist = sqrtf(dot(vv, vv) / dot(u, u));
-                if (dist < min_d)
-                    min_d = dist;
+                const float sq = dot(vv, vv) / dot(u, u);
+                if (sq < min_q)
+                    min_q = sq;
             }
         }
-        s.d_edge = min_d;
+        if (min_q < __int_as_float(0x7f800000))
+            s.d_edge = sqrtf(min_q);
         break;
     }
     case FR_GEOM_POLYGON: {  // fresnel/cpu/GeometryPolygon.cc:146-230

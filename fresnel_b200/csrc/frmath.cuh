@@ -336,8 +336,17 @@ FR_HD C3 brdf_diffuse(const Mat& m, V3 l, V3 v, V3 n, C3 sc)
     return diffuse_term(m, base_color(m, sc), ndotl, ndotv, ldoth) * (1.0f - m.metal);
 }
 
-// Material::brdf_specular (Material.h:153-218)
-FR_HD C3 brdf_specular(const Mat& m, V3 l, V3 v, V3 n, C3 sc, float half_angle)
+// The light's half angle as brdf_specular takes it, through the tangent it enters by (0: no light
+// size).
+FR_HD float light_spread(float half_angle)
+{
+    if (half_angle > 0.99f * PI_F / 2.0f)
+        half_angle = 0.99f * PI_F / 2.0f;
+    return half_angle > 0.0f ? 0.5f * htan(half_angle) : -1.0f;
+}
+
+// Material::brdf_specular (Material.h:153-218); spread: light_spread of the light's half angle
+FR_HD C3 brdf_specular(const Mat& m, V3 l, V3 v, V3 n, C3 sc, float spread)
 {
     float ndotv = dot(n, v);
     if (ndotv <= 0)
@@ -351,10 +360,8 @@ FR_HD C3 brdf_specular(const Mat& m, V3 l, V3 v, V3 n, C3 sc, float half_angle)
     float alpha = m.roughness * m.roughness;
     float alpha_sq = alpha * alpha;
     float D = ggx_d(alpha_sq, ndoth);
-    if (half_angle > 0.99f * PI_F / 2.0f)
-        half_angle = 0.99f * PI_F / 2.0f;
-    if (half_angle > 0.0f) {
-        float ap = alpha + 0.5f * htan(half_angle);
+    if (spread >= 0.0f) {
+        float ap = alpha + spread;
         if (ap > 1.0f)
             ap = 1.0f;
         D = D * alpha_sq / (ap * ap);
@@ -364,11 +371,12 @@ FR_HD C3 brdf_specular(const Mat& m, V3 l, V3 v, V3 n, C3 sc, float half_angle)
     return D * F * V;
 }
 
-// tangent frame of the importance samplers; `fabs(float) > 0.999` compares in double
+// tangent frame of the importance samplers; the reference's `fabs(float) > 0.999` compares in
+// double: true from the float 0.999f (just above 0.999) on
 FR_HD void tangent_frame(V3 n, V3& tx, V3& ty)
 {
     V3 up = v3(0, 0, 1.0f);
-    if (double(fabsf(n.z)) > 0.999)
+    if (fabsf(n.z) >= 0.999f)
         up = v3(1.0f, 0, 0);
     tx = cross(up, n);
     tx = div_recip(tx, sqrtf(dot(tx, tx)));

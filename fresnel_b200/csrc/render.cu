@@ -692,8 +692,9 @@ __global__ void __launch_bounds__(256) k_path_extend_grid_refill(FrameParams P, 
 
 // Representative-point area-light shading of one preview sample
 // (fresnel/cpu/TracerDirect.cc:120-200).
+// spread: light_spread of each light's half angle (block_spread).
 __device__ __forceinline__ C3 preview_shade(const FrameParams& P, const GeomDev& g,
-                                            const Surface& sf, V3 dir)
+                                            const Surface& sf, V3 dir, const float* spread)
 {
     V3 n = div_each(sf.Ng, sqrtf(dot(sf.Ng, sf.Ng)));
     V3 v = div_recip(-dir, sqrtf(dot(dir, dir)));
@@ -718,10 +719,22 @@ __device__ __forceinline__ C3 preview_shade(const FrameParams& P, const GeomDev&
         if (ndotl >= 0.0f)
             f_d = brdf_diffuse(m, l, v, n, sf.color) * ndotl;
         if (dot(n, r) >= 0.0f)
-            f_s = brdf_specular(m, r, v, n, sf.color, half) * dot(n, r);
+            f_s = brdf_specular(m, r, v, n, sf.color, spread[li]) * dot(n, r);
         c = c + (f_d + f_s) * PI_F * P.lights.color[li];
     }
     return c;
+}
+
+// The lights' spreads, once per block instead of once per sample and light (a tangent in double
+// precision).
+__device__ __forceinline__ const float* block_spread(const FrameParams& P)
+{
+    __shared__ float spread[4];
+    const uint32_t t = threadIdx.x + threadIdx.y * blockDim.x;
+    if (t < P.lights.n)
+        spread[t] = light_spread(P.lights.theta[t]);
+    __syncthreads();
+    return spread;
 }
 
 // The frame's rays (one path each), added by the launch's first thread.
@@ -741,6 +754,7 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
     uint32_t j = blockIdx.y * blockDim.y + threadIdx.y;
     bool valid = (i < P.w) && (j < P.h);
     const uint32_t ns = aa_n * aa_n;
+    const float* spread = block_spread(P);
     TraceCount tc;
     if (valid) {
         uint32_t p = j * P.w + i;
@@ -754,7 +768,7 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
             if (h.geom != MISS) {
                 const GeomDev& g = P.scene.geoms[h.geom];
                 Surface sf = hit_surface(g, h.prim, o, d, 0.0f);
-                c = preview_shade(P, g, sf, d);
+                c = preview_shade(P, g, sf, d, spread);
                 a = 1.0f;
             }
             if (hits)
@@ -776,8 +790,9 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
 // and 8x8 anti-aliasing): lane l of a group traces samples l, l + G, ... of its pixel,
 // so that a warp's rays are a few pixels' own jittered samples, which walk the same cells and
 // nodes, where k_preview's warp holds 32 pixels whose sample loops run side by side.  Each round
-// of G samples is summed in sample order (every lane reads its group's G colours by shuffles), so
-// the pixel is the same float sum as k_preview's; the hit ids go to the same places.
+// of G samples is summed in sample order (lanes 0-3 of the group each add one channel of the G
+// colours, left in shared memory), so the pixel is the same float sum as k_preview's; the hit ids go
+// to the same places.
 template <int WIDTH, uint32_t MASK, uint32_t G, bool LISTS = false>
 __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa_n, uint2* hits)
 {
@@ -788,12 +803,15 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
     const uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const bool valid = p < P.w * P.h;  // uniform within a group
     const uint32_t ns = aa_n * aa_n;   // a multiple of G
+    const float* spread = block_spread(P);
+    __shared__ float4 colours[PATH_BLOCK / 32][32];
+    float* const sums = reinterpret_cast<float*>(colours[threadIdx.x >> 5]);
     TraceCount tc;
     if (valid) {
         const uint32_t j = p / P.w, i = p - j * P.w;
         const uint2* list = LISTS ? pixel_list(P, i, j) : nullptr;
         const bool empty = LISTS && list_empty(list);
-        float avg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float avg = 0.0f;  // lanes 0-3 of the group: red, green, blue, alpha
         for (uint32_t base = 0; base < ns; base += G) {
             const uint32_t sample = base + gl;
             V3 o, d;
@@ -813,23 +831,27 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
             if (h.geom != MISS) {
                 const GeomDev& g = P.scene.geoms[h.geom];
                 Surface sf = hit_surface(g, h.prim, o, d, 0.0f);
-                c = preview_shade(P, g, sf, d);
+                c = preview_shade(P, g, sf, d, spread);
                 a = 1.0f;
             }
             if (hits)
                 hits[size_t(p) * ns + sample] =
                     make_uint2(h.geom == MISS ? 0u : h.geom + 1u, h.geom == MISS ? 0u : h.prim);
-            for (uint32_t k = 0; k < G; ++k) {
-                avg[0] += __shfl_sync(gmask, c.r, first + k);
-                avg[1] += __shfl_sync(gmask, c.g, first + k);
-                avg[2] += __shfl_sync(gmask, c.b, first + k);
-                avg[3] += __shfl_sync(gmask, a, first + k);
+            colours[threadIdx.x >> 5][lane] = make_float4(c.r, c.g, c.b, a);
+            __syncwarp(gmask);
+            if (gl < 4u) {
+#pragma unroll
+                for (uint32_t k = 0; k < G; ++k)
+                    avg += sums[4u * (first + k) + gl];
             }
+            __syncwarp(gmask);
         }
-        if (gl == 0u) {
-            const float q = 1.0f / float(ns);
-            write_pixel(P, p, avg[0] * q, avg[1] * q, avg[2] * q, avg[3] * q);
-        }
+        const float q = 1.0f / float(ns);
+        avg = avg * q;
+        const float r = __shfl_sync(gmask, avg, first), gr = __shfl_sync(gmask, avg, first + 1u),
+                    b = __shfl_sync(gmask, avg, first + 2u), al = __shfl_sync(gmask, avg, first + 3u);
+        if (gl == 0u)
+            write_pixel(P, p, r, gr, b, al);
     }
     flush_block(tc, P.stats + 3);
     count_preview(P, ns);
