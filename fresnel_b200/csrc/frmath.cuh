@@ -778,6 +778,21 @@ FR_HD uint32_t srgb_pack(float r, float g, float b, float a)
     uint32_t out = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
+#ifdef __CUDA_ARCH__
+        // The power in double precision decides only the byte it rounds to, and single precision
+        // (a few units in the last place: 3e-4 of a byte at most) gives the same one unless it
+        // lies that close to the next byte's threshold, which 1 value in 250 does
+        // (1M-sphere Preview 1080p 4.89 -> 4.54 ms, 4k cubes 4.70 -> 4.41).
+        if (x[k] >= 0.0031308f && x[k] <= 1.0f) {
+            const float v = ((1.0f + 0.055f) * exp2f(log2f(x[k]) * (1.0f / 2.4f)) - 0.055f) * 255.0f
+                            + 0.5f;
+            const float w = floorf(v);
+            if (v - w > 2e-3f && v - w < 1.0f - 2e-3f) {
+                out |= uint32_t(w) << (8 * k);
+                continue;
+            }
+        }
+#endif
         float y = (x[k] < 0.0031308f) ? 12.92f * x[k]
                                       : (1.0f + 0.055f) * hpow(x[k], 1.0f / 2.4f) - 0.055f;
         if (y > 1.0f)
