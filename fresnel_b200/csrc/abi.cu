@@ -367,9 +367,23 @@ struct fr_batch {
     int exec_width = 0;
     uint32_t exec_mask = 0;
     cudaStream_t capture = nullptr;
+    // renders of a wave side by side over packed queues (render_packed)
+    static constexpr int LANES = 32;
+    cudaStream_t lane[LANES] = {};
+    cudaEvent_t lane_ev[LANES] = {}, begin = nullptr;  // a lane's work is done; a wave may begin
+    DevArray<uint32_t> ctrs;
+    DevArray<uint2> lists;
     fr_batch_stats stats{};
     ~fr_batch()
     {
+        for (int k = 0; k < LANES; ++k) {
+            if (lane_ev[k])
+                cudaEventDestroy(lane_ev[k]);
+            if (lane[k])
+                cudaStreamDestroy(lane[k]);
+        }
+        if (begin)
+            cudaEventDestroy(begin);
         if (exec)
             cudaGraphExecDestroy(exec);
         if (capture)
@@ -1028,6 +1042,7 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
     P.linear = tr->linear.ptr;
     P.srgb = tr->srgb.ptr;
     P.stats = tr->stats.ptr;
+    P.tests = tr->stats.ptr + 3;
     return P;
 }
 
@@ -1042,25 +1057,36 @@ bool flat_layer(const GridDev& G) { return G.nx <= 1 || G.ny <= 1 || G.nz <= 1; 
 constexpr size_t WAVE_MIN_SLOTS = 1u << 21;
 constexpr uint32_t WAVE_TAIL_RAYS = 3u << 19;
 
-// Builds the frame's pixel lists on the stream and puts them into P where they apply and
-// `samples` camera rays per pixel pay for them.
-void prepare_lists(fr_device* dev, FrameParams& P, uint32_t samples)
+// Whether the frame gets pixel lists: where they apply and `samples` camera rays per pixel pay for
+// them.
+bool lists_wanted(const fr_device* dev, const FrameParams& P, uint32_t samples)
 {
-    if (!dev->pixel_lists || !lists_possible(P) ||
-        (dev->pixel_lists == 2 && !lists_pay(P, samples)))
-        return;
-    if (dev->lists.reserve(pixel_list_words(P)) != cudaSuccess) {
-        cudaGetLastError();  // no memory for them: the walk needs none
-        return;
-    }
+    return dev->pixel_lists && lists_possible(P) &&
+           (dev->pixel_lists != 2 || lists_pay(P, samples));
+}
+
+// Builds the frame's pixel lists on the stream (pixel_list_words(P) at `at`) and puts them into P.
+void build_lists(FrameParams& P, uint2* at, cudaStream_t st)
+{
     // Long enough lists end a tile's walk early.  Over spheres 9 entries answer all but a few
     // rays, and a walk for 15 costs more than those rays' own walks (200k spheres 1024x768, 16
     // samples: 2.95 ms a frame at 15, 2.85 at 8, 2.97 at 6; flat above 64 samples); over parts a
     // ray's own walk is expensive and the lists take all they hold (cubes Preview 5.8 ms at 15,
     // 6.6 at 11).
     P.list_enough = P.scene.grid.parts ? 15u : 9u;
-    launch_pixel_lists(P, dev->lists.ptr, dev->stream);
-    P.lists = dev->lists.ptr;
+    launch_pixel_lists(P, at, st);
+    P.lists = at;
+}
+
+void prepare_lists(fr_device* dev, FrameParams& P, uint32_t samples)
+{
+    if (!lists_wanted(dev, P, samples))
+        return;
+    if (dev->lists.reserve(pixel_list_words(P)) != cudaSuccess) {
+        cudaGetLastError();  // no memory for them: the walk needs none
+        return;
+    }
+    build_lists(P, dev->lists.ptr, dev->stream);
 }
 
 fr_status check_status(fr_device* dev)
@@ -2458,6 +2484,134 @@ fr_status fr_tracer_reset_stats(fr_tracer* t)
 // ---------------------------------------------------------------------------------------------
 // Batched path renders
 // ---------------------------------------------------------------------------------------------
+}  // extern "C"
+
+namespace {
+
+// Path slots per render from which a batch's renders go over packed queues, up to 32 at a time on
+// streams of their own, instead of through the batch's graph, whose fused kernels find every
+// path's render by a search and read its scene through memory.  Side by side the renders fill
+// each other's ends: 8 images of 20k spheres 384x384, 16 samples, take 5.44 ms one after another,
+// 4.39 two at a time, 4.05 together (graph 4.90); 5 images of 39M slots 28.1, 26.5 and 26.1
+// (43.0); 12 images of 3.7M slots with 4 light samples 22.8 (30.2).  Images whose longest path
+// outlasts all else must all run at once (10 dense ones of 600k slots: 23.0 ms eight at a time,
+// 19.0 together, graph 18.7).  Below the line the launches cost more: 590k slots 0.86 (1.01), 294k
+// 1.78 (1.87), but with several light samples, whose paths the tail follows one after another,
+// 810k slots 3.63 (3.36) and 263k 5.50 (4.60).
+constexpr size_t BATCH_WAVE_SLOTS = 1u << 19;
+constexpr size_t BATCH_WAVE_SLOTS_LIGHTS = 1u << 21;
+// Paths left that a render's tail kernel follows; the others' kernels fill the chip beside it, so
+// it starts later than WAVE_TAIL_RAYS (4.27 ms at 1.5M for the 8 images, 4.13 at 390k).
+constexpr uint32_t BATCH_TAIL_RAYS = 3u << 17;
+
+bool packed_pays(const fr_device* dev, const std::vector<WaveJob>& jobs)
+{
+    if (!dev->wave || dev->fuse_shade != 1 || dev->tail_after < 0)
+        return false;
+    size_t slots = 0, line = 0;
+    for (const WaveJob& J : jobs) {
+        const FrameParams& P = J.P;
+        if (P.scene.grid.n_cells == 0 || flat_layer(P.scene.grid) || P.refill || P.packet ||
+            P.persistent)
+            return false;
+        slots += padded_pixels(P.w, P.h, P.tile_log2) * P.batch;
+        line += P.light_samples > 1 ? BATCH_WAVE_SLOTS_LIGHTS : BATCH_WAVE_SLOTS;
+    }
+    return slots >= line;
+}
+
+// What the packed renders need beside the batch's path state; false when there is no memory for
+// it (the graph needs none of it).
+bool packed_room(fr_batch* b, const std::vector<WaveJob>& jobs,
+                 const std::vector<uint32_t>& wave_first, size_t slots)
+{
+    size_t words = 0;
+    int lanes = 0;
+    for (size_t w = 0; w + 1 < wave_first.size(); ++w) {
+        lanes = int(std::min<size_t>(fr_batch::LANES,
+                                     std::max<size_t>(lanes, wave_first[w + 1] - wave_first[w])));
+        size_t n = 0;
+        for (uint32_t j = wave_first[w]; j < wave_first[w + 1]; ++j)
+            if (lists_wanted(b->dev, jobs[j].P, jobs[j].P.batch))
+                n += pixel_list_words(jobs[j].P);
+        words = std::max(words, n);
+    }
+    cudaError_t e = b->ctrs.reserve(4 * jobs.size());
+    for (const WaveJob& J : jobs)
+        if (J.P.light_samples > 1 && e == cudaSuccess)
+            e = b->path.reserve_records(slots);
+    if (e == cudaSuccess && !b->begin)
+        e = cudaEventCreateWithFlags(&b->begin, cudaEventDisableTiming);
+    for (int k = 0; k < lanes && e == cudaSuccess; ++k) {
+        if (!b->lane[k])
+            e = cudaStreamCreateWithFlags(&b->lane[k], cudaStreamNonBlocking);
+        if (e == cudaSuccess && !b->lane_ev[k])
+            e = cudaEventCreateWithFlags(&b->lane_ev[k], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess && words)
+        e = b->lists.reserve(words);
+    if (e != cudaSuccess)
+        cudaGetLastError();
+    return e == cudaSuccess;
+}
+
+// Every wave's renders, LANES of them at a time: each has its part of the path state, queue
+// counters and pixel lists of its own, and no length is read back: the passes before the tail
+// follow from the render's slots (a pass ends about half of the paths).
+cudaError_t render_packed(fr_batch* b, std::vector<WaveJob>& jobs,
+                          const std::vector<uint32_t>& wave_first, uint64_t& launched)
+{
+    fr_device* dev = b->dev;
+    cudaStream_t st = dev->stream;
+    cudaError_t e = cudaMemsetAsync(b->ctrs.ptr, 0, 4 * sizeof(uint32_t) * jobs.size(), st);
+    for (size_t w = 0; w + 1 < wave_first.size() && e == cudaSuccess; ++w) {
+        const uint32_t j0 = wave_first[w], j1 = wave_first[w + 1];
+        e = cudaEventRecord(b->begin, st);
+        const int used = int(std::min<size_t>(fr_batch::LANES, j1 - j0));
+        for (int k = 0; k < used && e == cudaSuccess; ++k)
+            e = cudaStreamWaitEvent(b->lane[k], b->begin, 0);
+        size_t words = 0;
+        for (uint32_t j = j0; j < j1 && e == cudaSuccess; ++j) {
+            cudaStream_t ls = b->lane[int(j - j0) % used];
+            FrameParams P = jobs[j].P;
+            P.tests = &b->ctl.ptr->box_tests;
+            if (lists_wanted(dev, P, P.batch)) {
+                build_lists(P, b->lists.ptr + words, ls);
+                words += pixel_list_words(P);
+                ++launched;
+            }
+            PathState S = b->path.state(P.light_samples > 1).from(jobs[j].slot_base);
+            S.ctr = b->ctrs.ptr + 4 * size_t(j);
+            launch_path_primary_shade(P, S, true, ls);
+            int q = 0;
+            size_t left = padded_pixels(P.w, P.h, P.tile_log2) * P.batch;
+            do {
+                launch_wave_trace(P, S, q, dev->shape, ls);
+                launch_wave_shade(P, S, q, dev->shape, ls);
+                launched += 2;
+                q ^= 1;
+                left /= 2;
+            } while (left / 2 > BATCH_TAIL_RAYS);
+            launch_wave_tail(P, S, q, dev->shape, ls);
+            launch_path_fold(P, S, ls);
+            launched += 3;
+            e = cudaGetLastError();
+        }
+        for (int k = 0; k < used; ++k) {  // the batch's stream goes on when the wave is done
+            cudaError_t x = cudaEventRecord(b->lane_ev[k], b->lane[k]);
+            if (x == cudaSuccess)
+                x = cudaStreamWaitEvent(st, b->lane_ev[k], 0);
+            if (e == cudaSuccess)
+                e = x;
+        }
+    }
+    return e;
+}
+
+}  // namespace
+
+extern "C" {
+
 fr_status fr_batch_create(fr_device* dev, fr_batch** out)
 {
     FR_CHECK_NULL(dev);
@@ -2679,11 +2833,12 @@ fr_status fr_batch_render(fr_batch* b)
     FR_CUDA(cudaMemcpyAsync(b->ctl.ptr, b->h_ctl, sizeof(BatchCtl), cudaMemcpyHostToDevice, st),
             "uploading the batch plan");
 
-    if (b->exec && (moved || b->exec_width != width || b->exec_mask != mask)) {
+    const bool packed = packed_pays(dev, jobs) && packed_room(b, jobs, wave_first, cap);
+    if (b->exec && (moved || (!packed && (b->exec_width != width || b->exec_mask != mask)))) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
     }
-    if (!b->exec) {
+    if (!b->exec && !packed) {
         BatchDev B;
         B.jobs = b->jobs.ptr;
         B.wave_first = b->wave_first.ptr;
@@ -2701,7 +2856,9 @@ fr_status fr_batch_render(fr_batch* b)
     FR_CUDA(cudaEventCreate(&e0), "batch timing");
     FR_CUDA(cudaEventCreate(&e1), "batch timing");
     cudaEventRecord(e0, st);
-    cudaError_t le = cudaGraphLaunch(b->exec, st);
+    uint64_t launched = 0;
+    cudaError_t le = packed ? render_packed(b, jobs, wave_first, launched)
+                            : cudaGraphLaunch(b->exec, st);
     cudaEventRecord(e1, st);
     if (le == cudaSuccess)
         le = cudaMemcpyAsync(b->h_ctl, b->ctl.ptr, sizeof(BatchCtl), cudaMemcpyDeviceToHost, st);
@@ -2718,13 +2875,15 @@ fr_status fr_batch_render(fr_batch* b)
     const BatchCtl& c = *b->h_ctl;
     b->stats.renders += uint32_t(b->items.size());
     b->stats.waves += uint32_t(waves.size());
-    b->stats.graph_launches += 1;
+    b->stats.graph_launches += packed ? 0 : 1;
     b->stats.shade_extend_pairs += c.pairs;
     // fused grid waves: begin, primary, 3 queue clears, 2 bounces, tail, fold, end;
     // otherwise per wave: begin, primary, fold, end, and per pass: 2 shade, 2 extend, 1
     // condition; 1 start
-    if (b->exec_mask == MASK_GRID_FUSED || b->exec_mask == MASK_GRID_PARTS_FUSED ||
-        b->exec_mask == MASK_GRID_PARTS_NO_MESH_FUSED)
+    if (packed)
+        b->stats.kernel_launches += launched;
+    else if (b->exec_mask == MASK_GRID_FUSED || b->exec_mask == MASK_GRID_PARTS_FUSED ||
+             b->exec_mask == MASK_GRID_PARTS_NO_MESH_FUSED)
         b->stats.kernel_launches += 1 + 10 * uint64_t(waves.size());
     else
         b->stats.kernel_launches += 1 + 4 * uint64_t(waves.size()) + 5 * c.pairs;

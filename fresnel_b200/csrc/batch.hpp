@@ -7,6 +7,9 @@
 // wave, a nested `while` node alternates shade and extend until the wave's queue is empty.
 // Loop state lives in device memory, so the graph is captured once and relaunched for any plan
 // that fits its buffers.
+//
+// Waves of long renders over grids run beside the graph instead (abi.cu, render_packed): each
+// render's packed-queue kernels (wave.cu) on a stream of its own over its part of the path state.
 #ifndef FR_BATCH_HPP
 #define FR_BATCH_HPP
 

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) k_path_primary(FrameParams P, PathState S
         slot = g;
         push = primary_ray<WIDTH, MASK>(P, S, it, slot, tc);
     }
-    const uint32_t at = push_block(S, 1, push, tc, P.stats + 3);
+    const uint32_t at = push_block(S, 1, push, tc, P.tests);
     if (push)
         st_cs(S.queue[1] + at, slot);
     count_primary(P, g);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_primary_shade(
     TraceCount tc;
     if (it.valid)
         push = primary_shade<WIDTH, MASK, LISTS, REC>(P, S, it, g, tc, L);
-    const uint32_t at = push_block(S, 0, push, tc, P.stats + 3);
+    const uint32_t at = push_block(S, 0, push, tc, P.tests);
     if (push) {
         if constexpr (REC)
             store_record(S, 0, at, L);
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256) k_path_primary_persistent(FrameParams P, 
     TraceCount tc;
     uint32_t n_rays = 0;
     persistent_trace<MASK>(P, src, primary_items(P.w, P.h, P.batch, P.tile_log2), S.ctr + 3, tc, n_rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
     flush_rays(P, n_rays, true);
 }
 
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256) k_path_extend_persistent(FrameParams P, P
     TraceCount tc;
     uint32_t n_rays = 0;
     persistent_trace<MASK>(P, src, S.ctr[q], S.ctr + 2, tc, n_rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
     flush_rays(P, n_rays, false);
 }
 
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256) k_path_extend(FrameParams P, PathState S,
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(P.stats + 0, (unsigned long long)count);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // Extension rays traced and shaded at once (device option "fuse_shade"): the rays of queue q are
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_bounce(FramePa
         }
         push_queue(S, q ^ 1, push, p);
     }
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // The tail of a wavefront's bounces in one launch (sphere-grid scenes): once the early bounces
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_path_tail(FramePara
         rays += __shfl_xor_sync(0xffffffffu, rays, off);
     if (lane == 0 && rays)
         atomicAdd(P.stats + 0, rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(256) k_path_extend_refill(FrameParams P, PathS
         rays += __shfl_xor_sync(0xffffffffu, rays, off);
     if (lane == 0 && rays)
         atomicAdd(P.stats + 0, rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // Extension rays through the sphere grid with per-lane refill (device option "refill"): a lane
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(256) k_path_extend_grid_refill(FrameParams P, 
         rays += __shfl_xor_sync(0xffffffffu, rays, off);
     if (lane == 0 && rays)
         atomicAdd(P.stats + 0, rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // Representative-point area-light shading of one preview sample
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(256) k_preview(FrameParams P, uint32_t aa_n, u
         float q = 1.0f / float(ns);
         write_pixel(P, p, avg[0] * q, avg[1] * q, avg[2] * q, avg[3] * q);
     }
-    flush_block(tc, P.stats + 3);
+    flush_block(tc, P.tests);
     count_preview(P, ns);
 }
 
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
         if (gl == 0u)
             write_pixel(P, p, r, gr, b, al);
     }
-    flush_block(tc, P.stats + 3);
+    flush_block(tc, P.tests);
     count_preview(P, ns);
 }
 

@@ -38,7 +38,8 @@ struct FrameParams {
     C3 hl_color;
     float4* linear;     // [h][w] running mean, linear RGBA
     uint32_t* srgb;     // [h][w] RGBA8
-    unsigned long long* stats;  // [0] rays, [1] paths, [2] dropped, [3] box tests, [4] prim tests
+    unsigned long long* stats;  // [0] rays, [1] paths, [2] dropped samples
+    unsigned long long* tests;  // [0] box tests, [1] primitive tests
 };
 
 // Wavefront state of the path tracer (structure of arrays, one entry per path slot; a batch of
@@ -61,6 +62,29 @@ struct PathState {
     float4* rec_d[2];
     float4* rec_a[2];
     uint32_t* ctr;      // [0], [1] queue lengths, [2] extend and [3] primary work counters
+
+    // The state of the slots from n on (with the same counters).
+    PathState from(size_t n) const
+    {
+        PathState S = *this;
+        S.prim_o += n;
+        S.prim_d += n;
+        S.prim_hit += n;
+        S.ray_o += n;
+        S.ray_d += n;
+        S.att += n;
+        S.result += n;
+        S.ls_depth += n;
+        S.hit += n;
+        S.sample += n;
+        for (int q = 0; q < 2; ++q) {
+            S.queue[q] += n;
+            S.rec_o[q] += n;
+            S.rec_d[q] += n;
+            S.rec_a[q] += n;
+        }
+        return S;
+    }
 };
 
 struct LaunchShape {

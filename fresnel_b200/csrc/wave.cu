@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256, Walk::DEFERS ? 3 : 4) k_wave_trace(FrameP
                 W.resolve(P, PATH_TNEAR);
         }
     }
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 // The record i of queue q as a lane to shade (its hit still to be set).
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(256, fused_blocks(MASK)) k_wave_tail(FramePara
         rays += __shfl_xor_sync(0xffffffffu, rays, off);
     if (lane == 0 && rays)
         atomicAdd(P.stats + 0, rays);
-    flush_counts(tc, P.stats + 3);
+    flush_counts(tc, P.tests);
 }
 
 constexpr uint32_t NO_MESH = MASK_GRID_PARTS_NO_MESH & MASK_ALL;

@@ -379,7 +379,9 @@ typedef struct fr_batch_stats {
     uint32_t waves;               /* wavefronts (renders that fit the path state together) */
     uint64_t graph_launches;
     uint64_t graph_captures;
-    uint64_t kernel_launches;     /* kernels executed inside the graphs */
+    uint64_t kernel_launches;     /* kernels executed, inside the graphs or beside them (renders
+                                     of half a million path slots and more run on streams of
+                                     their own instead of in the graph) */
     uint64_t shade_extend_pairs;  /* device-side loop passes (two bounces each) */
     uint64_t box_tests, prim_tests;
     float last_ms;                /* device time of the last fr_batch_render */

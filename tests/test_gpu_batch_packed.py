@@ -1,0 +1,78 @@
+"""Batches whose renders go over packed queues side by side against the batch's graph.
+
+Both follow the same paths with the same arithmetic, so images and ray counts must be equal bit
+for bit: more renders than run at once, renders of several sizes, one and several light samples,
+a tracer that takes part twice and a wavefront too small for all (the renders then come in several
+waves, each with a share of the samples), camera rays answered by pixel lists, and grids over
+parts.
+"""
+
+import numpy
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _scenes(dev):
+    import fresnel_b200 as fresnel
+    from fresnel_b200 import workloads
+    scenes = []
+    for seed, n in ((1, 4000), (2, 900)):
+        rng = numpy.random.default_rng(seed)
+        scene = fresnel.Scene(dev, lights=fresnel.light.cloudy())
+        g = fresnel.geometry.Sphere(scene, position=rng.uniform(-9, 9, (n, 3)).astype(numpy.float32),
+                                    radius=0.6, outline_width=0.02 * seed)
+        g.color[:] = rng.uniform(0.2, 1, (n, 3))
+        g.material = fresnel.material.Material(primitive_color_mix=1.0, roughness=0.5,
+                                               spec_trans=0.1)
+        scene.camera = fresnel.camera.Orthographic.fit(scene)
+        scenes.append(scene)
+    scenes.append(workloads.config3(dev, scale=0.01))
+    return scenes
+
+
+CASES = {  # (scene, w, h, samples, light samples) per render, option path_slots, pixel_lists
+    "many": ([(0, 131, 97, 45, 1), (1, 300, 200, 9, 1)] * 17 + [(0, 257, 129, 20, 1)], None, 2),
+    "lights": ([(0, 256, 200, 45, 2), (1, 301, 190, 40, 3)], None, 2),
+    "parts": ([(2, 256, 256, 12, 1), (0, 256, 200, 16, 1), (2, 190, 130, 40, 1)], None, 2),
+    "lists": ([(0, 256, 200, 18, 1), (2, 256, 256, 17, 1), (1, 300, 200, 16, 1)], None, 1),
+    "waves": ([(0, 256, 256, 40, 1), (1, 256, 256, 24, 1), (0, 300, 200, 50, 1)], 1 << 21, 1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_packed_batch_gives_the_graphs_images(gpu_device, name):
+    import fresnel_b200 as fresnel
+    renders, slots, lists = CASES[name]
+    option = gpu_device._device.setOption
+    before = gpu_device._device.getOption("path_slots")
+    scenes = _scenes(gpu_device)
+    got = []
+    try:
+        if slots:
+            option("path_slots", slots)
+        option("pixel_lists", lists)
+        for wave in (1, 0):
+            option("wave", wave)
+            batch = fresnel.tracer.PathBatch(gpu_device)
+            tracers = []
+            for i, (k, w, h, spp, ls) in enumerate(renders):
+                t = fresnel.tracer.Path(gpu_device, w, h)
+                t.seed = 3 + i
+                batch.add(t, scenes[k], samples=spp, light_samples=ls)
+                tracers.append(t)
+            if name == "waves":
+                batch.add(tracers[1], scenes[0], samples=30, reset=False)
+            batch.render()
+            assert (batch.stats["graph_launches"] == 0) == bool(wave)
+            assert (batch.stats["waves"] > 1) == (name == "waves")
+            got.append([(t.linear_output[:].copy(), t.output[:].copy(),
+                         t._tracer.getStats()["rays"]) for t in tracers])
+        for (image, srgb, rays), (image0, srgb0, rays0) in zip(*got):
+            numpy.testing.assert_array_equal(image, image0)
+            numpy.testing.assert_array_equal(srgb, srgb0)
+            assert rays == rays0
+    finally:
+        option("wave", 1)
+        option("pixel_lists", 2)
+        option("path_slots", before)
