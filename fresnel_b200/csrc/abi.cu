@@ -2493,11 +2493,11 @@ namespace {
 // path's render by a search and read its scene through memory.  Side by side the renders fill
 // each other's ends: 8 images of 20k spheres 384x384, 16 samples, take 5.44 ms one after another,
 // 4.39 two at a time, 4.05 together (graph 4.90); 5 images of 39M slots 28.1, 26.5 and 26.1
-// (43.0); 12 images of 3.7M slots with 4 light samples 22.8 (30.2).  Images whose longest path
+// (43.0); 11 images of 4.2M slots with 4 light samples 31.6 (41.6).  Images whose longest path
 // outlasts all else must all run at once (10 dense ones of 600k slots: 23.0 ms eight at a time,
 // 19.0 together, graph 18.7).  Below the line the launches cost more: 590k slots 0.86 (1.01), 294k
-// 1.78 (1.87), but with several light samples, whose paths the tail follows one after another,
-// 810k slots 3.63 (3.36) and 263k 5.50 (4.60).
+// 1.78 (1.87), but with several light samples, which take as many more passes, 1.7M slots 12.1
+// (12.1) and 667k 2.85 (2.50).
 constexpr size_t BATCH_WAVE_SLOTS = 1u << 19;
 constexpr size_t BATCH_WAVE_SLOTS_LIGHTS = 1u << 21;
 // Paths left that a render's tail kernel follows; the others' kernels fill the chip beside it, so
@@ -2557,7 +2557,10 @@ bool packed_room(fr_batch* b, const std::vector<WaveJob>& jobs,
 
 // Every wave's renders, LANES of them at a time: each has its part of the path state, queue
 // counters and pixel lists of its own, and no length is read back: the passes before the tail
-// follow from the render's slots (a pass ends about half of the paths).
+// follow from the render's slots (a pass ends about half of the paths) and its light samples (a
+// slot's next one begins where the last ended, so the queue stays long for about as many passes:
+// 7 images of 2.1M slots with 13 light samples 54.8 ms without those passes, 43.8 with them, graph
+// 60.3).
 cudaError_t render_packed(fr_batch* b, std::vector<WaveJob>& jobs,
                           const std::vector<uint32_t>& wave_first, uint64_t& launched)
 {
@@ -2583,16 +2586,16 @@ cudaError_t render_packed(fr_batch* b, std::vector<WaveJob>& jobs,
             PathState S = b->path.state(P.light_samples > 1).from(jobs[j].slot_base);
             S.ctr = b->ctrs.ptr + 4 * size_t(j);
             launch_path_primary_shade(P, S, true, ls);
-            int q = 0;
-            size_t left = padded_pixels(P.w, P.h, P.tile_log2) * P.batch;
-            do {
-                launch_wave_trace(P, S, q, dev->shape, ls);
-                launch_wave_shade(P, S, q, dev->shape, ls);
-                launched += 2;
-                q ^= 1;
-                left /= 2;
-            } while (left / 2 > BATCH_TAIL_RAYS);
-            launch_wave_tail(P, S, q, dev->shape, ls);
+            uint32_t passes = std::min(P.light_samples, 32u);  // (launches are bounded)
+            for (size_t left = padded_pixels(P.w, P.h, P.tile_log2) * P.batch;
+                 left / 4 > BATCH_TAIL_RAYS; left /= 2)
+                ++passes;
+            for (uint32_t q = 0; q < passes; ++q) {
+                launch_wave_trace(P, S, int(q & 1u), dev->shape, ls);
+                launch_wave_shade(P, S, int(q & 1u), dev->shape, ls);
+            }
+            launched += 2 * passes;
+            launch_wave_tail(P, S, int(passes & 1u), dev->shape, ls);
             launch_path_fold(P, S, ls);
             launched += 3;
             e = cudaGetLastError();
