@@ -575,7 +575,7 @@ def run_batch_bench(args, world, rank, barrier_max, barrier_sum, clock_index, em
         "gpu_launches": int(launches),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm if achieved else None, "traffic": None,
-                     "peak_source": peak_kind, "kernel": "whole batch graph (all kernels)",
+                     "peak_source": peak_kind, "kernel": "whole batch (all kernels)",
                      "bytes_per_ray": bpr,
                      "bytes_per_ray_basis": "sphere grids walked, engine counters"
                      if grid else "structures walked, engine counters"},
@@ -789,6 +789,9 @@ def main():
         # without shade launches each bounce traces and shades in one kernel
         primary_name = "k_path_primary_shade" if dd.getOption("fuse_shade") else "k_path_primary"
         ext_name = "k_path_bounce" if st["shade_launches"] == 0 else "k_path_extend"
+        if st.get("grid", 0) and st["shade_launches"] and dd.getOption("wave"):
+            # packed queues: a pass traces and one shades, then one tail launch does both
+            ext_name = "k_wave_trace+k_wave_tail"
         if ext_name == "k_path_bounce" and dd.getOption("tail") >= 0:
             # the fused bounces of a wavefront: bounce launches, then one tail launch that
             # follows every remaining path (timed together as the extension kernels)

@@ -162,8 +162,9 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *   "bvh_width"     2 or 4: binary or 4-wide tree traversed by the renderers (default 4)
  *   "leaf_max"      largest leaf the SAH collapse may form (1..16, default 2)
  *   "c_trav"        SAH cost of one node visit relative to one primitive test (default 1)
- *   "path_slots"    path slots traced together by the path tracer, 144 bytes each
- *                   (default 134217728: 18.4 GB; a batch takes at most what it can fill)
+ *   "path_slots"    path slots traced together by the path tracer, 144 bytes each (192 with
+ *                   several light samples over packed queues, see "wave"; default 134217728:
+ *                   18.4 GB; a batch takes at most what it can fill)
  *   "persistent"    1: 4-wide traversal in persistent warps with per-lane refill;
  *                   0: one ray per thread (default)
  *   "builder"       0: LBVH (Karras hierarchy, default); 1: PLOC (locally-ordered clustering)
@@ -212,11 +213,12 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   separate passes over queues of whole path records (at least 2M path
  *                   slots), the tracing with per-lane refill; 0: fused bounces as below.  The
  *                   same images in both cases.
- *   "tail"          fused sphere-grid bounces: after this many bounce launches per wavefront
- *                   (0..64, default 1), one persistent launch follows every remaining path to
- *                   its end (a lane takes the next path once its own ends), with no queue
- *                   read-back; -1: a bounce launch per bounce until the queue is empty.  The
- *                   same images in every case.
+ *   "tail"          fused bounces over a grid, and passes over a tree of spheres with one light
+ *                   sample: after this many bounce launches (passes) per wavefront (0..64,
+ *                   default 1), one persistent launch follows every remaining path to its end
+ *                   (a lane takes the next path once its own ends), with no queue read-back;
+ *                   -1: a launch per bounce until the queue is empty, and no packed queues
+ *                   ("wave").  The same images in every case.
  * Setting an option marks every BVH of the device's scenes for rebuild when it changes the
  * tree.  Unknown names or out-of-range values return FR_ERR_INVALID. */
 FR_API fr_status fr_device_set_option(fr_device* dev, const char* name, double value);
