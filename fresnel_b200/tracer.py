@@ -116,8 +116,9 @@ class PathBatch:
 
     ``add(tracer, scene, samples, reset=True, light_samples=1)`` queues what
     ``tracer.sample(scene, samples, reset, light_samples)`` renders; ``render()`` traces every
-    queued render in one CUDA graph launch. The renders share wavefronts, so many small frames
-    keep the GPU as busy as one large frame. Afterwards each tracer holds the image its own
+    queued render, small ones in one CUDA graph launch and long ones over grids side by side on
+    streams. The renders share wavefronts, so many small frames keep the GPU as busy as one large
+    frame. Afterwards each tracer holds the image its own
     ``sample`` call would have produced. Tracers and scenes can differ in size and content but
     must belong to the batch's device.
     """
@@ -163,5 +164,6 @@ class PathBatch:
     @property
     def stats(self):
         """Counters over the batch's lifetime: renders, waves, graph launches and captures,
-        kernels run inside the graphs, device-side loop passes, traversal tests, device ms."""
+        kernels run (inside the graphs or beside them), device-side loop passes, traversal tests,
+        device ms."""
         return self._batch.getStats()

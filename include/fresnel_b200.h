@@ -371,7 +371,8 @@ FR_API fr_status fr_tracer_render_path_static(fr_tracer* tr, fr_scene* scene,
  * No counterpart in the reference, which renders one Tracer.Path call at a time.  A batch
  * queues path renders of any tracers, scenes and image sizes on one device and traces them
  * together: their pixel samples share wavefronts and kernel launches, and the whole batch is
- * one CUDA graph launch (device-side loops over waves and bounces, no host round trips).  Each
+ * one CUDA graph launch (device-side loops over waves and bounces, no host round trips), or, for
+ * long renders over grids, packed-queue kernels of every render on streams of the batch.  Each
  * render's output equals what fr_tracer_render_path gives for the same arguments.  Renders of
  * one tracer are traced in the order they were added.  Tracers and scenes must stay alive until
  * fr_batch_render returns; fr_batch_render keeps the queue (fr_batch_clear empties it). */
