@@ -26,6 +26,34 @@ using namespace fr;
 
 namespace {
 
+// fr_debug_fail_allocations: this thread's next `after` allocations succeed, the `count` ones after
+// them fail, `failed` did.
+thread_local struct {
+    uint32_t after = 0, count = 0, failed = 0;
+} g_alloc_failures;
+
+}  // namespace
+
+namespace fr {
+
+cudaError_t device_alloc(void** out, size_t bytes)
+{
+    auto& f = g_alloc_failures;
+    if (f.count && f.after) {
+        --f.after;
+    } else if (f.count) {
+        --f.count;
+        ++f.failed;
+        *out = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
+    return cudaMalloc(out, bytes);
+}
+
+}  // namespace fr
+
+namespace {
+
 thread_local std::string g_error;
 
 fr_status fail(fr_status s, const std::string& msg)
@@ -738,6 +766,7 @@ fr_status prepare_grid(fr_scene* sc, fr_tracer* tr, int kind, uint32_t gi,
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, dev->stream);
+    sc->grid.bounds = false;
     cudaError_t e;
     if (kind == 1) {
         const fr_geometry* g = parts[0];
@@ -790,7 +819,6 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
     std::vector<uint64_t> key;
     uint32_t gi = 0;
     std::vector<fr_geometry*> grid_parts;
-    bool grid_built = false;
     const int kind = grid_candidate(sc, key, gi, &grid_parts);
     if (kind == 0) {
         sc->use_grid = false;
@@ -799,7 +827,6 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
         fr_status s = prepare_grid(sc, tr, kind, gi, grid_parts, key);
         if (s != FR_OK)
             return s;
-        grid_built = true;
     }
     const std::vector<fr_geometry*> parts =
         sc->use_grid ? std::vector<fr_geometry*>() : combined_parts(sc, key);
@@ -905,20 +932,33 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
         }
         sc->table_dirty = false;
     }
-    if (grid_built && sc->use_grid && sc->grid.parts) {
-        GridBuffers& G = sc->grid;
-        FR_CUDA(G.ref_bound.reserve(G.n_refs), "allocating a grid");
-        SceneDev d;
-        std::memset(&d, 0, sizeof(d));
-        d.geoms = sc->table.ptr;
-        d.n_geoms = uint32_t(sc->geoms.size());
-        d.leaf_data = G.ref_data.ptr;
-        d.leaf_geom = G.ref_geom.ptr;
-        d.order = G.ref_prim.ptr;
-        launch_part_bounds(d, G.n_refs, G.ref_bound.ptr, dev->stream);
-        FR_CUDA(cudaGetLastError(), "building a grid");
-    }
     return FR_OK;
+}
+
+// The spheres around the references of a prepared scene's grid over parts (GridDev::ref_bound),
+// which only the packed-queue kernels read: made by the first render through those after each
+// build of the grid, so that renders through other kernels (flat layers, Preview, short
+// wavefronts) neither allocate nor fill them.  False when there is no memory for them (the
+// fused kernels need none).  A sphere grid needs none either.
+bool have_part_bounds(fr_scene* sc)
+{
+    GridBuffers& G = sc->grid;
+    if (!G.parts || G.bounds)
+        return true;
+    if (G.ref_bound.reserve(G.n_refs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    SceneDev d;
+    std::memset(&d, 0, sizeof(d));
+    d.geoms = sc->table.ptr;
+    d.n_geoms = uint32_t(sc->geoms.size());
+    d.leaf_data = G.ref_data.ptr;
+    d.leaf_geom = G.ref_geom.ptr;
+    d.order = G.ref_prim.ptr;
+    launch_part_bounds(d, G.n_refs, G.ref_bound.ptr, sc->dev->stream);
+    G.bounds = cudaGetLastError() == cudaSuccess;
+    return G.bounds;
 }
 
 FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p, bool preview,
@@ -958,7 +998,6 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
         d.cell_start = G.cell_start.ptr;
         d.ref_sphere = G.ref_sphere.ptr;
         d.ref_prim = G.ref_prim.ptr;
-        d.ref_bound = G.ref_bound.ptr;
         d.parts = G.parts ? 1u : 0u;
         if (G.parts) {  // the references read as a combined tree's leaf slots
             for (fr_geometry* g : sc->geoms)
@@ -1949,7 +1988,10 @@ fr_status fr_tracer_render_path(fr_tracer* t, fr_scene* sc, const fr_render_para
     // extension rays over packed queues (wave.cu)
     bool wave = t->dev->wave && t->dev->fuse_shade == 1 && t->dev->tail_after >= 0 && !P.refill &&
                 !P.packet && P.scene.grid.n_cells != 0 && !flat_layer(P.scene.grid) &&
-                padded_pixels(t->w, t->h, t->dev->tile_log2) * batch >= WAVE_MIN_SLOTS;
+                padded_pixels(t->w, t->h, t->dev->tile_log2) * batch >= WAVE_MIN_SLOTS &&
+                have_part_bounds(sc);
+    if (wave)
+        P.scene.grid.ref_bound = sc->grid.ref_bound.ptr;
     if (wave && light_samples > 1 &&
         t->dev->path.reserve_records(padded_pixels(t->w, t->h, t->dev->tile_log2) * batch) !=
             cudaSuccess) {
@@ -2441,6 +2483,14 @@ fr_status fr_tracer_read_primary_hits(fr_tracer* t, uint32_t* host, size_t nbyte
     return FR_OK;
 }
 
+fr_status fr_debug_fail_allocations(uint32_t after, uint32_t count, uint32_t* failed)
+{
+    if (failed)
+        *failed = g_alloc_failures.failed;
+    g_alloc_failures = {after, count, 0};
+    return FR_OK;
+}
+
 fr_status fr_debug_traversal_compare(fr_scene* sc, const float* rays, uint32_t n, uint32_t* out)
 {
     FR_CHECK_NULL(sc);
@@ -2520,11 +2570,16 @@ bool packed_pays(const fr_device* dev, const std::vector<WaveJob>& jobs)
     return slots >= line;
 }
 
-// What the packed renders need beside the batch's path state; false when there is no memory for
-// it (the graph needs none of it).
-bool packed_room(fr_batch* b, const std::vector<WaveJob>& jobs,
+// What the packed renders need beside the batch's path state (`scenes`: each job's); false when
+// there is no memory for it (the graph needs none of it).
+bool packed_room(fr_batch* b, std::vector<WaveJob>& jobs, const std::vector<fr_scene*>& scenes,
                  const std::vector<uint32_t>& wave_first, size_t slots)
 {
+    for (size_t j = 0; j < jobs.size(); ++j) {
+        if (!have_part_bounds(scenes[j]))
+            return false;
+        jobs[j].P.scene.grid.ref_bound = scenes[j]->grid.ref_bound.ptr;
+    }
     size_t words = 0;
     int lanes = 0;
     for (size_t w = 0; w + 1 < wave_first.size(); ++w) {
@@ -2773,6 +2828,7 @@ fr_status fr_batch_render(fr_batch* b)
 
     // render table
     std::vector<WaveJob> jobs;
+    std::vector<fr_scene*> job_scene;
     std::vector<uint32_t> wave_first, wave_items, wave_pixels;
     int width = 4;
     uint32_t mask = 0;
@@ -2803,6 +2859,7 @@ fr_status fr_batch_render(fr_batch* b)
             if (slot > 0xFFFFFFFFull || item > 0xFFFFFFFFull || pixel > 0xFFFFFFFFull)
                 return fail(FR_ERR_INVALID, "a batch wave exceeds 2^32 slots");
             jobs.push_back(J);
+            job_scene.push_back(it.sc);
         }
         wave_items.push_back(uint32_t(item));
         wave_pixels.push_back(uint32_t(pixel));
@@ -2836,7 +2893,7 @@ fr_status fr_batch_render(fr_batch* b)
     FR_CUDA(cudaMemcpyAsync(b->ctl.ptr, b->h_ctl, sizeof(BatchCtl), cudaMemcpyHostToDevice, st),
             "uploading the batch plan");
 
-    const bool packed = packed_pays(dev, jobs) && packed_room(b, jobs, wave_first, cap);
+    const bool packed = packed_pays(dev, jobs) && packed_room(b, jobs, job_scene, wave_first, cap);
     if (b->exec && (moved || (!packed && (b->exec_width != width || b->exec_mask != mask)))) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;

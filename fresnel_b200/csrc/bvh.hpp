@@ -10,6 +10,9 @@
 namespace fr {
 
 // A growable device allocation: reserve() only reallocates when the request exceeds capacity.
+// cudaMalloc of the arrays below, with the failures fr_debug_fail_allocations asks for.
+cudaError_t device_alloc(void** out, size_t bytes);
+
 template <class T> struct DevArray {
     T* ptr = nullptr;
     size_t cap = 0;  // elements
@@ -20,7 +23,7 @@ template <class T> struct DevArray {
         release();
         if (n == 0)
             return cudaSuccess;
-        cudaError_t e = cudaMalloc((void**)&ptr, n * sizeof(T));
+        cudaError_t e = device_alloc((void**)&ptr, n * sizeof(T));
         if (e != cudaSuccess) {
             ptr = nullptr;
             cap = 0;

@@ -15,6 +15,7 @@ struct GridBuffers {
     DevArray<float4> ref_data;       // parts grid, per reference: 2 float4 of the primitive's
                                      // record (laid out as a combined tree's leaf slot)
     DevArray<float4> ref_bound;      // parts grid, per reference: a sphere around it (engine.cuh)
+    bool bounds = false;             // ref_bound holds those of the present references
     DevArray<uint32_t> ref_geom;     // parts grid, per reference: scene geometry index
     DevArray<uint32_t> prim_count;   // build temporaries kept between builds: cells per primitive
     DevArray<uint32_t> prim_offset;  // and their exclusive prefix sum

@@ -914,6 +914,13 @@ PYBIND11_MODULE(_gpu, m)
         return n;
     });
 
+    m.def("debugFailAllocations", [](unsigned after, unsigned count) {
+        // how many the setting before this one failed
+        uint32_t failed = 0;
+        check(fr_debug_fail_allocations(after, count, &failed));
+        return failed;
+    });
+
     py::class_<DeviceH, std::shared_ptr<DeviceH>>(m, "Device")
         .def(py::init<const std::string&, int>())
         .def("describe", &DeviceH::describe)

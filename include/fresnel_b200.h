@@ -413,6 +413,12 @@ FR_API fr_status fr_batch_get_stats(const fr_batch* batch, fr_batch_stats* out);
 FR_API fr_status fr_debug_traversal_compare(fr_scene* scene, const float* rays, uint32_t n,
                                             uint32_t* out);
 
+/* Lets device allocations fail, for tests of what follows (no counterpart in the reference): of those
+ * the calling thread makes from now on, the first `after` are tried as ever and the next `count`
+ * report that there is no memory without being tried; count 0: none.  failed (may be null)
+ * receives how many the calling thread's previous setting failed. */
+FR_API fr_status fr_debug_fail_allocations(uint32_t after, uint32_t count, uint32_t* failed);
+
 /* Runs the engine's device Philox4x32-10 and cuRAND's curand_Philox4x32_10 on n inputs
  * in[i] = (ctr0, ctr1, ctr2, ctr3, key0, key1) (host arrays; outputs n x 4 words each).
  * No counterpart in the reference: Random123's known-answer vectors are not in its tree, and
