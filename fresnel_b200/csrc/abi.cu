@@ -392,6 +392,7 @@ struct fr_batch {
     PathBuffers path;
     BatchCtl* h_ctl = nullptr;  // pinned
     cudaGraphExec_t exec = nullptr;
+    bool moved = false;  // an array's address is no longer the graph's (also when growing it failed)
     int exec_width = 0;
     uint32_t exec_mask = 0;
     cudaStream_t capture = nullptr;
@@ -2872,12 +2873,11 @@ fr_status fr_batch_render(fr_batch* b)
     if (mask == 0)
         mask = MASK_SPHERES;  // empty scenes: every ray misses
 
-    bool moved = false;
-    FR_CUDA(grow(b->jobs, jobs.size(), moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_first, wave_first.size(), moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_items, wave_items.size(), moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_pixels, wave_pixels.size(), moved), "allocating the batch plan");
-    FR_CUDA(b->path.reserve(cap, &moved), "allocating the batch path state");
+    FR_CUDA(grow(b->jobs, jobs.size(), b->moved), "allocating the batch plan");
+    FR_CUDA(grow(b->wave_first, wave_first.size(), b->moved), "allocating the batch plan");
+    FR_CUDA(grow(b->wave_items, wave_items.size(), b->moved), "allocating the batch plan");
+    FR_CUDA(grow(b->wave_pixels, wave_pixels.size(), b->moved), "allocating the batch plan");
+    FR_CUDA(b->path.reserve(cap, &b->moved), "allocating the batch path state");
 
     cudaStream_t st = dev->stream;
     FR_CUDA(cudaMemcpyAsync(b->jobs.ptr, jobs.data(), jobs.size() * sizeof(WaveJob),
@@ -2894,10 +2894,11 @@ fr_status fr_batch_render(fr_batch* b)
             "uploading the batch plan");
 
     const bool packed = packed_pays(dev, jobs) && packed_room(b, jobs, job_scene, wave_first, cap);
-    if (b->exec && (moved || (!packed && (b->exec_width != width || b->exec_mask != mask)))) {
+    if (b->exec && (b->moved || (!packed && (b->exec_width != width || b->exec_mask != mask)))) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
     }
+    b->moved = false;
     if (!b->exec && !packed) {
         BatchDev B;
         B.jobs = b->jobs.ptr;
@@ -2962,12 +2963,7 @@ fr_status fr_batch_reserve(fr_batch* b, size_t slots)
     fr_status s = use_device(b->dev);
     if (s != FR_OK)
         return s;
-    bool moved = false;
-    FR_CUDA(b->path.reserve(slots, &moved), "allocating the batch path state");
-    if (moved && b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        b->exec = nullptr;
-    }
+    FR_CUDA(b->path.reserve(slots, &b->moved), "allocating the batch path state");
     return FR_OK;
 }
 

@@ -83,3 +83,57 @@ def test_render_after_a_failed_allocation(gpu_device, name):
     assert raised > 10
     # bounding spheres; they and three record arrays; three record arrays and the lists; none
     assert served == {"parts": 1, "parts_lights": 4, "spheres_lists": 4, "parts_short": 0}[name]
+
+
+def _batch(dev, batch, scenes, spp, lights):
+    tracers = []
+    for i, scene in enumerate(scenes):
+        t = fresnel.tracer.Path(dev, *SIZE)
+        t.seed = 4 + i
+        batch.add(t, scene, samples=spp, light_samples=lights)
+        tracers.append(t)
+    batch.render()
+    return [t.linear_output[:].copy() for t in tracers]
+
+
+@pytest.mark.parametrize("wave", [0, 1])
+def test_batch_after_a_failed_allocation(gpu_device, wave):
+    """A small batch (captured as a graph), then larger ones whose allocations fail one after
+    another, each followed by the small one again: its graph must not run over arrays that moved.
+    """
+    def setup():
+        dev = fresnel.Device(mode="gpu")
+        dev._device.setOption("wave", wave)
+        dev._device.setOption("pixel_lists", 1)
+        scenes = [_parts(dev), _parts(dev), _spheres(dev)]
+        for i, s in enumerate(scenes):
+            s.background_color = (0.1 * i, 0.2, 0.3)
+        return dev, scenes, fresnel.tracer.PathBatch(dev)
+
+    dev, scenes, batch = setup()
+    small = _batch(dev, batch, scenes[:1], 2, 1)
+    large = _batch(dev, batch, scenes, 100, 2)
+    raised = 0
+    for k in range(200):
+        dev, scenes, batch = setup()
+        _batch(dev, batch, scenes[:1], 2, 1)
+        _fail(k + 9)  # (after the images and counters of the three tracers)
+        try:
+            images = _batch(dev, batch, scenes, 100, 2)
+        except RuntimeError as e:
+            assert "memory" in str(e)
+            images = None
+            raised += 1
+        failed = _fail(0, 0)
+        if images is not None:
+            for a, b in zip(images, large):
+                numpy.testing.assert_array_equal(a, b)
+        if not failed:
+            break
+        for a, b in zip(_batch(dev, batch, scenes[:1], 2, 1), small):
+            numpy.testing.assert_array_equal(a, b)
+        for a, b in zip(_batch(dev, batch, scenes, 100, 2), large):
+            numpy.testing.assert_array_equal(a, b)
+    else:
+        pytest.fail("the batch allocates without end")
+    assert raised > 10
