@@ -76,3 +76,30 @@ def test_packed_batch_gives_the_graphs_images(gpu_device, name):
         option("wave", 1)
         option("pixel_lists", 2)
         option("path_slots", before)
+
+
+@pytest.mark.parametrize("lights,height,packed", [(1, 40.0, True), (2, 40.0, True),
+                                                  (1, 4000.0, True), (2, 4000.0, False)])
+def test_batches_that_miss_take_the_graph(gpu_device, lights, height, packed):
+    """With several light samples a packed render's passes are worth their launches only where
+    enough camera rays hit: the same batch with the scene filling the image, and as a few pixels
+    in its middle."""
+    import fresnel_b200 as fresnel
+    scene = _scenes(gpu_device)[0]
+    scene.camera = fresnel.camera.Orthographic(position=(60, 50, 70), look_at=(0, 0, 0),
+                                               up=(0, 1, 0), height=height)
+    option = gpu_device._device.setOption
+    got = []
+    try:
+        for wave in (1, 0):
+            option("wave", wave)
+            batch = fresnel.tracer.PathBatch(gpu_device)
+            t = fresnel.tracer.Path(gpu_device, 256, 256)
+            t.seed = 8
+            batch.add(t, scene, samples=36, light_samples=lights)
+            batch.render()
+            assert (batch.stats["graph_launches"] == 0) == (packed and wave == 1)
+            got.append(t.linear_output[:].copy())
+    finally:
+        option("wave", 1)
+    numpy.testing.assert_array_equal(got[0], got[1])
