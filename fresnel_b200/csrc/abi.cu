@@ -159,7 +159,15 @@ struct PathBuffers {
             e = rec_d.reserve(n);
         if (e == cudaSuccess)
             e = rec_a.reserve(n);
+        if (e != cudaSuccess)
+            release_records();
         return e;
+    }
+    void release_records()
+    {
+        rec_o.release();
+        rec_d.release();
+        rec_a.release();
     }
     PathState state(bool lights = false) const
     {
@@ -191,6 +199,8 @@ struct PathBuffers {
 
 struct fr_tracer;
 
+struct fr_batch;
+
 struct fr_device {
     int ordinal = 0;
     cudaStream_t stream = nullptr;
@@ -221,6 +231,7 @@ struct fr_device {
     int tail_after = 1;                    // fused bounce launches before the tail kernel (-1: none)
     float grid_cells_per_prim = 1.5f;      // grid cells per sphere
     std::vector<fr_scene*> scenes;         // to mark BVHs stale when a build option changes
+    std::vector<fr_batch*> batches;
     void* static_path = nullptr;           // this device's copy of g_static_path (looked up once)
     PathBuffers path;                      // wavefront state shared by the device's tracers
     uint32_t* h_count = nullptr;           // pinned word for queue-length readbacks
@@ -488,6 +499,50 @@ bool planes_within(const float* origins, const float* normals, uint32_t n, float
     return vertices >= 4;
 }
 
+// Frees the device's optional arrays, which renders keep from one call to the next and can do without
+// (pixel lists, the packed kernels' second record queue and bounding spheres); false when it
+// holds none.
+bool give_back(fr_device* dev)
+{
+    bool any = false;
+    const auto drop = [&](auto& a) {
+        any = any || a.ptr;
+        a.release();
+    };
+    const auto records = [&](PathBuffers& p) {
+        any = any || p.rec_o.ptr;
+        p.release_records();
+    };
+    drop(dev->lists);
+    records(dev->path);
+    for (fr_batch* b : dev->batches) {
+        drop(b->lists);
+        records(b->path);
+    }
+    for (fr_scene* sc : dev->scenes) {
+        drop(sc->grid.ref_bound);
+        sc->grid.bounds = false;
+    }
+    return any;
+}
+
+// An allocation that a call cannot do without: when there is no memory for it, the optional arrays
+// go first.  (Made before a call takes any of those for itself.)
+template <class F> cudaError_t needed(fr_device* dev, F&& allocate)
+{
+    cudaError_t e = allocate();
+    if (e == cudaErrorMemoryAllocation && give_back(dev)) {
+        cudaGetLastError();
+        e = allocate();
+    }
+    return e;
+}
+
+template <class T> cudaError_t needed(fr_device* dev, DevArray<T>& a, size_t n)
+{
+    return needed(dev, [&] { return a.reserve(n); });
+}
+
 uint64_t g_generation = 0;  // source of fr_geometry::gen values (never repeats)
 
 void mark_moved(fr_geometry* g)
@@ -508,7 +563,7 @@ fr_status alloc_field(fr_geometry* g, int f)
     DevArray<float>* a = g->field(f, count);
     if (!a || count == 0)
         return FR_OK;
-    FR_CUDA(a->reserve(count), "allocating a geometry array");
+    FR_CUDA(needed(g->scene->dev, *a, count), "allocating a geometry array");
     FR_CUDA(cudaMemsetAsync(a->ptr, 0, count * sizeof(float), g->scene->dev->stream),
             "clearing a geometry array");
     return FR_OK;
@@ -723,9 +778,13 @@ fr_status build_combined(fr_scene* sc, fr_tracer* tr, const std::vector<fr_geome
     cudaEventRecord(e0, dev->stream);
     cudaError_t e = cudaErrorInvalidValue;
     if (refit)
-        e = refit_bvh(in, n, bp, sc->combined, dev->scratch, dev->status.ptr, dev->stream);
+        e = needed(dev, [&] {
+            return refit_bvh(in, n, bp, sc->combined, dev->scratch, dev->status.ptr, dev->stream);
+        });
     if (!refit || e == cudaErrorInvalidValue)
-        e = build_bvh(in, n, bp, sc->combined, dev->scratch, dev->status.ptr, dev->stream);
+        e = needed(dev, [&] {
+            return build_bvh(in, n, bp, sc->combined, dev->scratch, dev->status.ptr, dev->stream);
+        });
     cudaEventRecord(e1, dev->stream);
     cudaEventSynchronize(e1);
     float ms = 0.0f;
@@ -771,12 +830,16 @@ fr_status prepare_grid(fr_scene* sc, fr_tracer* tr, int kind, uint32_t gi,
     cudaError_t e;
     if (kind == 1) {
         const fr_geometry* g = parts[0];
-        e = build_grid(g->position.ptr, g->radius.ptr, g->n, gp, sc->grid, dev->scratch,
-                       dev->stream, sc->grid_report);
+        e = needed(dev, [&] {
+            return build_grid(g->position.ptr, g->radius.ptr, g->n, gp, sc->grid, dev->scratch,
+                              dev->stream, sc->grid_report);
+        });
     } else {
         uint32_t n = 0;
         const PartsInput in = parts_input(sc, parts, n, true);
-        e = build_grid(in, n, gp, sc->grid, dev->scratch, dev->stream, sc->grid_report);
+        e = needed(dev, [&] {
+            return build_grid(in, n, gp, sc->grid, dev->scratch, dev->stream, sc->grid_report);
+        });
     }
     cudaEventRecord(e1, dev->stream);
     cudaEventSynchronize(e1);
@@ -853,11 +916,15 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
                            same_params(g->bvh_bp, bp);
         cudaError_t e = cudaErrorInvalidValue;
         if (refit)
-            e = refit_bvh(in, g->bvh_prims(), bp, g->bvh, dev->scratch, dev->status.ptr,
-                          dev->stream);
+            e = needed(dev, [&] {
+                return refit_bvh(in, g->bvh_prims(), bp, g->bvh, dev->scratch, dev->status.ptr,
+                                 dev->stream);
+            });
         if (!refit || e == cudaErrorInvalidValue)
-            e = build_bvh(in, g->bvh_prims(), bp, g->bvh, dev->scratch, dev->status.ptr,
-                          dev->stream);
+            e = needed(dev, [&] {
+                return build_bvh(in, g->bvh_prims(), bp, g->bvh, dev->scratch, dev->status.ptr,
+                                 dev->stream);
+            });
         cudaEventRecord(e1, dev->stream);
         cudaEventSynchronize(e1);
         float ms = 0.0f;
@@ -925,7 +992,7 @@ fr_status prepare_scene(fr_scene* sc, fr_tracer* tr)
             d.outline = to_mat(g->outline);
         }
         if (!host.empty()) {
-            FR_CUDA(sc->table.reserve(host.size()), "allocating the geometry table");
+            FR_CUDA(needed(dev, sc->table, host.size()), "allocating the geometry table");
             FR_CUDA(cudaMemcpyAsync(sc->table.ptr, host.data(), host.size() * sizeof(GeomDev),
                                     cudaMemcpyHostToDevice, dev->stream),
                     "uploading the geometry table");
@@ -1151,8 +1218,8 @@ fr_status check_status(fr_device* dev)
 fr_status alloc_outputs(fr_tracer* tr, uint32_t w, uint32_t h)
 {
     size_t n = size_t(w) * h;
-    FR_CUDA(tr->linear.reserve(n), "allocating the linear output");
-    FR_CUDA(tr->srgb.reserve(n), "allocating the sRGB output");
+    FR_CUDA(needed(tr->dev, tr->linear, n), "allocating the linear output");
+    FR_CUDA(needed(tr->dev, tr->srgb, n), "allocating the sRGB output");
     FR_CUDA(cudaMemsetAsync(tr->linear.ptr, 0, n * sizeof(float4), tr->dev->stream), "clear");
     FR_CUDA(cudaMemsetAsync(tr->srgb.ptr, 0, n * sizeof(uint32_t), tr->dev->stream), "clear");
     tr->w = w;
@@ -1185,7 +1252,7 @@ uint32_t batch_size(const fr_tracer* tr, uint32_t remaining)
 fr_status alloc_path_state(fr_tracer* tr, uint32_t batch)
 {
     size_t n = padded_pixels(tr->w, tr->h, tr->dev->tile_log2) * batch;
-    FR_CUDA(tr->dev->path.reserve(n), "allocating the path state");
+    FR_CUDA(needed(tr->dev, [&] { return tr->dev->path.reserve(n); }), "allocating the path state");
     return FR_OK;
 }
 
@@ -1602,11 +1669,12 @@ fr_status fr_geometry_create_polyhedron(fr_scene* scene, const float* origins, c
         pl4[2 * size_t(i)] = make_float4(nn.x, nn.y, nn.z, -dot(nn, p));
         pl4[2 * size_t(i) + 1] = make_float4(p.x, p.y, p.z, 0.0f);
     }
-    cudaError_t e = use_device(scene->dev) == FR_OK ? g->planes.reserve(pl.size()) : cudaErrorUnknown;
+    cudaError_t e = use_device(scene->dev) == FR_OK ? needed(scene->dev, g->planes, pl.size())
+                                                    : cudaErrorUnknown;
     if (e == cudaSuccess)
         e = cudaMemcpy(g->planes.ptr, pl.data(), pl.size() * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
-        e = g->planes4.reserve(pl4.size());
+        e = needed(scene->dev, g->planes4, pl4.size());
     if (e == cudaSuccess)
         e = cudaMemcpy(g->planes4.ptr, pl4.data(), pl4.size() * sizeof(float4),
                        cudaMemcpyHostToDevice);
@@ -1668,13 +1736,14 @@ fr_status fr_geometry_create_mesh(fr_scene* scene, const float* vertices, uint32
             boxes[2 * size_t(f) + 1] = make_float4(hi[0] + pad, hi[1] + pad, hi[2] + pad, 0.0f);
         }
     }
-    cudaError_t e = use_device(scene->dev) == FR_OK ? g->vertices.reserve(size_t(n_vertices) * 3)
-                                                    : cudaErrorUnknown;
+    cudaError_t e = use_device(scene->dev) == FR_OK
+                        ? needed(scene->dev, g->vertices, size_t(n_vertices) * 3)
+                        : cudaErrorUnknown;
     if (e == cudaSuccess && n_vertices)
         e = cudaMemcpy(g->vertices.ptr, vertices, size_t(n_vertices) * 3 * sizeof(float),
                        cudaMemcpyHostToDevice);
     if (e == cudaSuccess && g->n_faces)
-        e = g->face_box.reserve(boxes.size());
+        e = needed(scene->dev, g->face_box, boxes.size());
     if (e == cudaSuccess && g->n_faces)
         e = cudaMemcpy(g->face_box.ptr, boxes.data(), boxes.size() * sizeof(float4),
                        cudaMemcpyHostToDevice);
@@ -1719,13 +1788,14 @@ fr_status fr_geometry_create_polygon(fr_scene* scene, const float* vertices, uin
     std::vector<float> q(size_t(n) * 4, 0.0f);
     for (uint32_t i = 0; i < n; ++i)
         q[4 * size_t(i)] = 1.0f;
-    cudaError_t e = use_device(scene->dev) == FR_OK ? g->vertices.reserve(size_t(n_vertices) * 2)
-                                                    : cudaErrorUnknown;
+    cudaError_t e = use_device(scene->dev) == FR_OK
+                        ? needed(scene->dev, g->vertices, size_t(n_vertices) * 2)
+                        : cudaErrorUnknown;
     if (e == cudaSuccess && n_vertices)
         e = cudaMemcpy(g->vertices.ptr, vertices, size_t(n_vertices) * 2 * sizeof(float),
                        cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
-        e = g->orientation.reserve(q.size());
+        e = needed(scene->dev, g->orientation, q.size());
     if (e == cudaSuccess && n)
         e = cudaMemcpy(g->orientation.ptr, q.data(), q.size() * sizeof(float),
                        cudaMemcpyHostToDevice);
@@ -1913,7 +1983,7 @@ fr_status fr_tracer_create(fr_device* dev, uint32_t w, uint32_t h, fr_tracer** o
     if (!t)
         return fail(FR_ERR_OUT_OF_MEMORY, "out of host memory");
     t->dev = dev;
-    cudaError_t e = t->stats.reserve(8);
+    cudaError_t e = needed(dev, t->stats, 8);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(t->stats.ptr, 0, 8 * sizeof(unsigned long long), dev->stream);
     if (e != cudaSuccess) {
@@ -2309,7 +2379,7 @@ fr_status fr_tracer_render_preview(fr_tracer* t, fr_scene* sc, const fr_render_p
     size_t nh = size_t(t->w) * t->h * aa_n * aa_n;
     uint2* hits = nullptr;
     if (hit_ids) {
-        FR_CUDA(t->preview_hits.reserve(nh), "allocating the hit-id buffer");
+        FR_CUDA(needed(t->dev, t->preview_hits, nh), "allocating the hit-id buffer");
         hits = t->preview_hits.ptr;
     }
     if (preview_groups(P, aa_n))
@@ -2364,7 +2434,7 @@ fr_status fr_tracer_histogram(fr_tracer* t, uint32_t* counts, size_t nbytes)
     fr_status s = use_device(t->dev);
     if (s != FR_OK)
         return s;
-    FR_CUDA(t->hist.reserve(size_t(HIST_BINS) * 4), "allocating the histogram");
+    FR_CUDA(needed(t->dev, t->hist, size_t(HIST_BINS) * 4), "allocating the histogram");
     cudaStream_t st = t->dev->stream;
     FR_CUDA(cudaMemsetAsync(t->hist.ptr, 0, nbytes, st), "clearing the histogram");
     launch_histogram(t->linear.ptr, t->w * t->h, t->hist.ptr, t->dev->num_sms, st);
@@ -2749,11 +2819,12 @@ fr_status fr_batch_create(fr_device* dev, fr_batch** out)
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
     if (e == cudaSuccess)
-        e = b->ctl.reserve(1);
+        e = needed(dev, b->ctl, 1);
     if (e != cudaSuccess) {
         delete b;
         return cuda_fail(e, "creating a batch");
     }
+    dev->batches.push_back(b);
     *out = b;
     return FR_OK;
 }
@@ -2762,6 +2833,8 @@ fr_status fr_batch_destroy(fr_batch* b)
 {
     if (!b)
         return FR_OK;
+    auto& v = b->dev->batches;
+    v.erase(std::remove(v.begin(), v.end(), b), v.end());
     cudaSetDevice(b->dev->ordinal);
     cudaStreamSynchronize(b->dev->stream);
     delete b;
@@ -2798,13 +2871,13 @@ fr_status fr_batch_add_path(fr_batch* b, fr_tracer* t, fr_scene* sc, const fr_re
 
 namespace {
 
-// Grow a batch buffer; reports whether its address changed (the graph then has to be redone).
-template <class T> cudaError_t grow(DevArray<T>& a, size_t n, bool& moved)
+// Grow a batch buffer, noting whether its address changed (the graph then has to be redone).
+template <class T> cudaError_t grow(fr_batch* b, DevArray<T>& a, size_t n)
 {
     T* old = a.ptr;
-    cudaError_t e = a.reserve(n);
+    cudaError_t e = needed(b->dev, a, n);
     if (a.ptr != old)
-        moved = true;
+        b->moved = true;
     return e;
 }
 
@@ -2937,11 +3010,12 @@ fr_status fr_batch_render(fr_batch* b)
     if (mask == 0)
         mask = MASK_SPHERES;  // empty scenes: every ray misses
 
-    FR_CUDA(grow(b->jobs, jobs.size(), b->moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_first, wave_first.size(), b->moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_items, wave_items.size(), b->moved), "allocating the batch plan");
-    FR_CUDA(grow(b->wave_pixels, wave_pixels.size(), b->moved), "allocating the batch plan");
-    FR_CUDA(b->path.reserve(cap, &b->moved), "allocating the batch path state");
+    FR_CUDA(grow(b, b->jobs, jobs.size()), "allocating the batch plan");
+    FR_CUDA(grow(b, b->wave_first, wave_first.size()), "allocating the batch plan");
+    FR_CUDA(grow(b, b->wave_items, wave_items.size()), "allocating the batch plan");
+    FR_CUDA(grow(b, b->wave_pixels, wave_pixels.size()), "allocating the batch plan");
+    FR_CUDA(needed(dev, [&] { return b->path.reserve(cap, &b->moved); }),
+            "allocating the batch path state");
 
     cudaStream_t st = dev->stream;
     FR_CUDA(cudaMemcpyAsync(b->jobs.ptr, jobs.data(), jobs.size() * sizeof(WaveJob),
@@ -3027,7 +3101,8 @@ fr_status fr_batch_reserve(fr_batch* b, size_t slots)
     fr_status s = use_device(b->dev);
     if (s != FR_OK)
         return s;
-    FR_CUDA(b->path.reserve(slots, &b->moved), "allocating the batch path state");
+    FR_CUDA(needed(b->dev, [&] { return b->path.reserve(slots, &b->moved); }),
+            "allocating the batch path state");
     return FR_OK;
 }
 

@@ -137,3 +137,41 @@ def test_batch_after_a_failed_allocation(gpu_device, wave):
     else:
         pytest.fail("the batch allocates without end")
     assert raised > 10
+
+
+def test_optional_arrays_make_room(gpu_device):
+    """Pixel lists and second record queues stay with a device and its batches between renders; an
+    allocation that then fails once succeeds without them, whichever it is."""
+    def run(k):
+        dev = fresnel.Device(mode="gpu")
+        dev._device.setOption("pixel_lists", 1)
+        scene = _spheres(dev)
+        t = fresnel.tracer.Path(dev, *SIZE)
+        t.seed = 9
+        t.sample(scene, 100, light_samples=2)
+        batch = fresnel.tracer.PathBatch(dev)
+        _batch(dev, batch, [scene], 100, 2)
+        if k is not None:
+            _fail(k)
+        parts = _parts(dev)  # every array of a scene, a larger image, more path slots, a batch
+        large = fresnel.tracer.Path(dev, 210, 170)
+        large.seed = 5
+        large.sample(parts, 70)
+        small = fresnel.tracer.Preview(dev, 64, 48, anti_alias=True)
+        small.render(parts)
+        images = [large.linear_output[:].copy(), small.linear_output[:].copy()]
+        images += _batch(dev, fresnel.tracer.PathBatch(dev), [parts, scene], 70, 1)
+        dev._device.setOption("accel", 0)  # trees
+        large.seed = 5
+        large.sample(parts, 3)
+        images.append(large.linear_output[:].copy())
+        return images, _fail(0, 0)
+
+    wanted, _ = run(None)
+    for k in range(200):
+        images, failed = run(k)
+        for a, b in zip(images, wanted):
+            numpy.testing.assert_array_equal(a, b)
+        if not failed:
+            break
+    assert 40 < k < 199
