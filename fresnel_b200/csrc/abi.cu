@@ -412,7 +412,8 @@ struct fr_batch {
     cudaStream_t lane[LANES] = {};
     cudaEvent_t lane_ev[LANES] = {}, begin = nullptr;  // a lane's work is done; a wave may begin
     DevArray<uint32_t> ctrs;
-    DevArray<uint2> lists;
+    DevArray<uint2> lists;       // every lane's pixel lists, one render's at a time,
+    size_t lists_at[LANES] = {};  // from here on
     fr_batch_stats stats{};
     ~fr_batch()
     {
@@ -2705,6 +2706,13 @@ bool packed_pays(const fr_device* dev, const std::vector<WaveJob>& jobs)
     return slots >= line && hits >= hits_line;
 }
 
+// Streams that the renders of a wave run on, one after another on each (render j of the wave on
+// stream j modulo their number).
+int wave_lanes(const std::vector<uint32_t>& wave_first, size_t wave)
+{
+    return int(std::min<size_t>(fr_batch::LANES, wave_first[wave + 1] - wave_first[wave]));
+}
+
 // What the packed renders need beside the batch's path state (`scenes`: each job's); false when
 // there is no memory for it (the graph needs none of it).
 bool packed_room(fr_batch* b, std::vector<WaveJob>& jobs, const std::vector<fr_scene*>& scenes,
@@ -2715,16 +2723,21 @@ bool packed_room(fr_batch* b, std::vector<WaveJob>& jobs, const std::vector<fr_s
             return false;
         jobs[j].P.scene.grid.ref_bound = scenes[j]->grid.ref_bound.ptr;
     }
-    size_t words = 0;
     int lanes = 0;
+    size_t lane_words[fr_batch::LANES] = {};
     for (size_t w = 0; w + 1 < wave_first.size(); ++w) {
-        lanes = int(std::min<size_t>(fr_batch::LANES,
-                                     std::max<size_t>(lanes, wave_first[w + 1] - wave_first[w])));
-        size_t n = 0;
+        const int used = wave_lanes(wave_first, w);
+        lanes = std::max(lanes, used);
         for (uint32_t j = wave_first[w]; j < wave_first[w + 1]; ++j)
-            if (lists_wanted(b->dev, jobs[j].P, jobs[j].P.batch))
-                n += pixel_list_words(jobs[j].P);
-        words = std::max(words, n);
+            if (lists_wanted(b->dev, jobs[j].P, jobs[j].P.batch)) {
+                size_t& n = lane_words[int(j - wave_first[w]) % used];
+                n = std::max(n, pixel_list_words(jobs[j].P));
+            }
+    }
+    size_t words = 0;
+    for (int k = 0; k < lanes; ++k) {
+        b->lists_at[k] = words;
+        words += lane_words[k];
     }
     cudaError_t e = b->ctrs.reserve(4 * jobs.size());
     for (const WaveJob& J : jobs)
@@ -2745,8 +2758,8 @@ bool packed_room(fr_batch* b, std::vector<WaveJob>& jobs, const std::vector<fr_s
     return e == cudaSuccess;
 }
 
-// Every wave's renders, LANES of them at a time: each has its part of the path state, queue
-// counters and pixel lists of its own, and no length is read back: the passes before the tail
+// Every wave's renders, LANES of them at a time: each has its part of the path state and queue
+// counters of its own, its lane's pixel lists are its own while it runs, and no length is read back: the passes before the tail
 // follow from the render's slots (a pass ends about half of the paths) and its light samples (a
 // slot's next one begins where the last ended, so the queue stays long for about as many passes:
 // 7 images of 2.1M slots with 13 light samples 54.8 ms without those passes, 43.8 with them, graph
@@ -2760,17 +2773,16 @@ cudaError_t render_packed(fr_batch* b, std::vector<WaveJob>& jobs,
     for (size_t w = 0; w + 1 < wave_first.size() && e == cudaSuccess; ++w) {
         const uint32_t j0 = wave_first[w], j1 = wave_first[w + 1];
         e = cudaEventRecord(b->begin, st);
-        const int used = int(std::min<size_t>(fr_batch::LANES, j1 - j0));
+        const int used = wave_lanes(wave_first, w);
         for (int k = 0; k < used && e == cudaSuccess; ++k)
             e = cudaStreamWaitEvent(b->lane[k], b->begin, 0);
-        size_t words = 0;
         for (uint32_t j = j0; j < j1 && e == cudaSuccess; ++j) {
-            cudaStream_t ls = b->lane[int(j - j0) % used];
+            const int k = int(j - j0) % used;
+            cudaStream_t ls = b->lane[k];
             FrameParams P = jobs[j].P;
             P.tests = &b->ctl.ptr->box_tests;
             if (lists_wanted(dev, P, P.batch)) {
-                build_lists(P, b->lists.ptr + words, ls);
-                words += pixel_list_words(P);
+                build_lists(P, b->lists.ptr + b->lists_at[k], ls);
                 ++launched;
             }
             PathState S = b->path.state(P.light_samples > 1).from(jobs[j].slot_base);

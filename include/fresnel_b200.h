@@ -209,7 +209,8 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   scene traced through a grid; 2 (default): where they are expected to pay
  *                   (at least 16 samples per pixel, 3 million camera rays, beams thinner than
  *                   the primitives).  The same images in every case.  The lists take 128
- *                   bytes per pixel of the largest image so far (265 MB at 1920x1080); they,
+ *                   bytes per pixel of the largest image so far (265 MB at 1920x1080), in a
+ *                   batch of each of up to 32 renders that run side by side; they,
  *                   and the second record queue of "wave", are kept between renders and given
  *                   back when another allocation of the device finds no memory.
  *   "wave"          1 (default): bounces of scenes traced through a grid trace and shade in

@@ -103,3 +103,28 @@ def test_batches_that_miss_take_the_graph(gpu_device, lights, height, packed):
     finally:
         option("wave", 1)
     numpy.testing.assert_array_equal(got[0], got[1])
+
+
+def test_packed_batch_lists_take_a_lane_each(gpu_device):
+    """The pixel lists of a batch's renders take memory for those that run at once (32 streams), not
+    for all of its renders."""
+    import torch
+    import fresnel_b200 as fresnel
+    dev = fresnel.Device(mode="gpu")
+    scene = _scenes(dev)[0]
+    batch = fresnel.tracer.PathBatch(dev)
+    tracers = [fresnel.tracer.Path(dev, 192, 192) for _ in range(96)]
+    images, free = [], []
+    for lists in (0, 1):
+        dev._device.setOption("pixel_lists", lists)
+        for i, t in enumerate(tracers):
+            t.seed = i
+            batch.add(t, scene, samples=15)
+        batch.render()
+        assert batch.stats["graph_launches"] == 0 and batch.stats["waves"] == lists + 1
+        images.append([t.linear_output[:].copy() for t in tracers])
+        free.append(torch.cuda.mem_get_info()[0])
+    for a, b in zip(*images):
+        numpy.testing.assert_array_equal(a, b)
+    # 32 lists of 128 bytes per pixel, and as much again for what else the second render may take
+    assert 0 < free[0] - free[1] < 2 * 32 * 128 * 192 * 192
