@@ -1219,8 +1219,23 @@ fr_status check_status(fr_device* dev)
 fr_status alloc_outputs(fr_tracer* tr, uint32_t w, uint32_t h)
 {
     size_t n = size_t(w) * h;
-    FR_CUDA(needed(tr->dev, tr->linear, n), "allocating the linear output");
-    FR_CUDA(needed(tr->dev, tr->srgb, n), "allocating the sRGB output");
+    const auto both = [&](size_t pixels) {
+        const cudaError_t e = needed(tr->dev, tr->linear, pixels);
+        return e == cudaSuccess ? needed(tr->dev, tr->srgb, pixels) : e;
+    };
+    const cudaError_t e = both(n);
+    if (e != cudaSuccess) {
+        // the old arrays may be gone: a tracer that had an image keeps one of that size, cleared,
+        // or else has none (check_params)
+        n = size_t(tr->w) * tr->h;
+        if (both(n) != cudaSuccess) {
+            tr->w = tr->h = 0;
+        } else if (n) {
+            cudaMemsetAsync(tr->linear.ptr, 0, n * sizeof(float4), tr->dev->stream);
+            cudaMemsetAsync(tr->srgb.ptr, 0, n * sizeof(uint32_t), tr->dev->stream);
+        }
+        return cuda_fail(e, "allocating the output images");
+    }
     FR_CUDA(cudaMemsetAsync(tr->linear.ptr, 0, n * sizeof(float4), tr->dev->stream), "clear");
     FR_CUDA(cudaMemsetAsync(tr->srgb.ptr, 0, n * sizeof(uint32_t), tr->dev->stream), "clear");
     tr->w = w;
@@ -1264,6 +1279,8 @@ fr_status check_params(const fr_tracer* tr, const fr_scene* sc, const fr_render_
     FR_CHECK_NULL(p);
     if (sc->dev != tr->dev)
         return fail(FR_ERR_INVALID, "Scene and Tracer devices do not match");
+    if (tr->w == 0)
+        return fail(FR_ERR_STATE, "the tracer has no image: there was no memory to resize it");
     return FR_OK;
 }
 
@@ -2906,6 +2923,9 @@ fr_status fr_batch_render(fr_batch* b)
     fr_device* dev = b->dev;
     if (b->items.empty())
         return FR_OK;
+    for (auto& it : b->items)  // (a tracer may have been resized since it was added)
+        if ((s = check_params(it.tr, it.sc, &it.params)) != FR_OK)
+            return s;
 
     // scenes: build what is stale (each scene once)
     std::vector<fr_scene*> scenes;

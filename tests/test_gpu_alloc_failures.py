@@ -175,3 +175,39 @@ def test_optional_arrays_make_room(gpu_device):
         if not failed:
             break
     assert 40 < k < 199
+
+
+@pytest.mark.parametrize("failures", [1, 2])
+def test_resize_that_finds_no_memory(gpu_device, failures):
+    """A tracer whose resize fails keeps an image of its old size; when there is no memory even for
+    that, it renders nothing until a resize succeeds."""
+    dev = fresnel.Device(mode="gpu")
+    scene = _spheres(dev)
+    for kind in (fresnel.tracer.Path, fresnel.tracer.Preview):
+        t = kind(dev, 64, 48)
+        t.seed = 3
+        t.render(scene)
+        image = t.linear_output[:].copy()
+        batch = fresnel.tracer.PathBatch(dev)
+        if kind is fresnel.tracer.Path:
+            batch.add(t, scene, samples=1)
+        _fail(0, failures)
+        with pytest.raises(RuntimeError, match="memory"):
+            t.resize(640, 480)
+        assert _fail(0, 0) == failures
+        if failures == 1:
+            assert not t.linear_output[:].any() and t.linear_output[:].shape == image.shape
+        else:
+            with pytest.raises(RuntimeError, match="no memory to resize"):
+                t.render(scene)
+            if kind is fresnel.tracer.Path:
+                with pytest.raises(RuntimeError, match="no memory to resize"):
+                    batch.render()
+                with pytest.raises(RuntimeError, match="no memory to resize"):
+                    batch.add(t, scene, samples=1)
+        t.resize(64, 48)
+        if kind is fresnel.tracer.Path:
+            t.reset()
+        t.seed = 3
+        t.render(scene)
+        numpy.testing.assert_array_equal(t.linear_output[:], image)
