@@ -618,6 +618,7 @@ BuildInput build_input(const fr_geometry* g)
     in.vertices = g->vertices.ptr;
     in.n_faces = g->n_faces;
     in.poly_radius = g->poly_radius;
+    in.bounded = g->bounded ? 1 : 0;
     in.instances = 0;
     return in;
 }
@@ -1063,6 +1064,8 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
         d.ihz = 1.0f / G.cell[2];
         d.geom = sc->grid_geom;
         d.n_valid = G.n_valid;
+        d.n_refs = G.n_refs;
+        d.n_odd = G.n_odd;
         d.mean_radius = G.mean_radius;
         d.cell_start = G.cell_start.ptr;
         d.ref_sphere = G.ref_sphere.ptr;

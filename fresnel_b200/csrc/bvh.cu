@@ -1334,28 +1334,43 @@ cudaError_t parts_boxes(const PartsInput& in, uint32_t n, float4* lo, float4* hi
 }
 
 namespace {
-// A reference's geometry word of a grid over parts: the geometry index with its type above it.
-__global__ void k_tag_types(PartsInput in, uint32_t n, uint32_t* geom)
+// A reference's geometry word of a grid over parts: the geometry index with its type above it; and
+// the count of gather_parts.
+__global__ void k_tag_types(PartsInput in, uint32_t n, const float4* data, uint32_t* geom,
+                            uint32_t* odd)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n)
-        return;
-    const uint32_t gi = geom[s];
-    uint32_t type = 0;
-    for (uint32_t p = 0; p < in.n_parts; ++p)
-        if (in.geom[p] == gi)
-            type = uint32_t(in.part[p].type);
-    geom[s] = gi | (type << PART_TYPE_SHIFT);
+    bool is_odd = false;
+    if (s < n) {
+        const uint32_t gi = geom[s];
+        uint32_t type = 0;
+        bool bounded = true;
+        for (uint32_t p = 0; p < in.n_parts; ++p)
+            if (in.geom[p] == gi) {
+                type = uint32_t(in.part[p].type);
+                bounded = in.part[p].bounded != 0;
+            }
+        geom[s] = gi | (type << PART_TYPE_SHIFT);
+        if (odd && (type == FR_GEOM_POLYHEDRON || type == FR_GEOM_MESH)) {
+            const float4 q = data[2 * size_t(s) + 1];
+            const float q2 = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+            is_odd = !bounded || !(fabsf(q2 - 1.0f) < UNIT_SLACK);
+        }
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, is_odd);
+    if (m && (threadIdx.x & 31u) == 0u)
+        atomicAdd(odd, uint32_t(__popc(m)));
 }
 }  // namespace
 
 cudaError_t gather_parts(const PartsInput& in, const uint32_t* prims, uint32_t total,
-                         float4* data, uint32_t* order, uint32_t* geom, cudaStream_t st)
+                         float4* data, uint32_t* order, uint32_t* geom, uint32_t* odd,
+                         cudaStream_t st)
 {
     if (total == 0)
         return cudaSuccess;
     k_gather<<<(total + 255) / 256, 256, 0, st>>>(in, total, prims, data, order, geom);
-    k_tag_types<<<(total + 255) / 256, 256, 0, st>>>(in, total, geom);
+    k_tag_types<<<(total + 255) / 256, 256, 0, st>>>(in, total, data, geom, odd);
     return cudaGetLastError();
 }
 

@@ -85,6 +85,7 @@ struct BuildInput {
     const float* vertices;
     uint32_t n_faces;
     float poly_radius;  // polyhedron / polygon: bounding radius about the position
+    int bounded;        // polyhedron: its surface lies within poly_radius
     int instances;      // mesh: one primitive per instance (grids over parts) instead of one
                         // per triangle (trees)
 };
@@ -145,10 +146,16 @@ cudaError_t parts_boxes(const PartsInput& in, uint32_t n, float4* lo, float4* hi
 // without reading the geometry table.
 constexpr uint32_t PART_TYPE_SHIFT = 24;
 
+// A squared quaternion norm further from 1 scales a polyhedron or mesh beyond its bounding radius.
+constexpr float UNIT_SLACK = 1e-3f;
+
 // For each of `total` references to primitives of `in` (combined numbering, prims[r]): its
 // leaf-slot record (2 float4 at data + 2 r), its index within its geometry and its geometry word.
+// *odd (device, zero before; null: not counted) receives the polyhedra and meshes among them whose
+// surface may lie outside their bounding radius.
 cudaError_t gather_parts(const PartsInput& in, const uint32_t* prims, uint32_t total,
-                         float4* data, uint32_t* order, uint32_t* geom, cudaStream_t st);
+                         float4* data, uint32_t* order, uint32_t* geom, uint32_t* odd,
+                         cudaStream_t st);
 
 // Build the BVH of n primitives (n == 0 leaves an empty tree).  Synchronises the stream once
 // to read back the node count.

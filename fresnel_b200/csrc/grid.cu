@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "fresnel_b200.h"
 #include "grid.hpp"
 
 namespace fr {
@@ -283,6 +284,7 @@ cudaError_t build_cells(const Src& src, uint32_t n, const Reasons& why, const Gr
     rep = GridReport();
     out.n_cells = 0;
     out.n_refs = 0;
+    out.n_odd = 0;
     vals_out = nullptr;
     total_out = 0;
     if (n == 0) {
@@ -511,18 +513,27 @@ cudaError_t build_grid(const PartsInput& in, uint32_t n, const GridParams& gp, G
                    (e = parts_boxes(in, n, out.box_lo.ptr, out.box_hi.ptr, st)) != cudaSuccess))
         return e;
     const uint32_t* vals = nullptr;
-    uint32_t total = 0;
+    uint32_t total = 0, odd = 0;
     e = build_cells(BoxSource{out.box_lo.ptr, out.box_hi.ptr}, n, PART_REASONS, gp, out, scratch,
                     st, rep, vals, total);
     if (e != cudaSuccess || vals == nullptr)
         return e;
     if ((e = out.ref_data.reserve(2 * size_t(total))) != cudaSuccess ||
         (e = out.ref_prim.reserve(total)) != cudaSuccess ||
-        (e = out.ref_geom.reserve(total)) != cudaSuccess ||
+        (e = out.ref_geom.reserve(size_t(total) + 1)) != cudaSuccess)
+        return e;
+    uint32_t* count = nullptr;  // of odd references, behind the geometry words
+    for (uint32_t p = 0; p < in.n_parts; ++p)
+        if (in.part[p].type == FR_GEOM_POLYHEDRON || in.part[p].type == FR_GEOM_MESH)
+            count = out.ref_geom.ptr + total;
+    if ((count && (e = cudaMemsetAsync(count, 0, sizeof(uint32_t), st)) != cudaSuccess) ||
         (e = gather_parts(in, vals, total, out.ref_data.ptr, out.ref_prim.ptr, out.ref_geom.ptr,
-                          st)) != cudaSuccess ||
+                          count, st)) != cudaSuccess ||
+        (count && (e = cudaMemcpyAsync(&odd, count, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                       st)) != cudaSuccess) ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return e;
+    out.n_odd = odd;
     out.parts = true;
     out.n_cells = uint32_t(uint64_t(out.dims[0]) * out.dims[1] * out.dims[2]);
     out.n_refs = total;

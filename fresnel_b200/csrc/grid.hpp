@@ -23,6 +23,7 @@ struct GridBuffers {
     DevArray<float4> box_hi;
     uint32_t n_cells = 0;            // 0: no grid
     uint32_t n_refs = 0;
+    uint32_t n_odd = 0;              // of them, those whose surface may lie outside their bounds
     float mean_radius = 0.0f;        // root of the mean cross-section / pi of the primitives
     uint32_t n_valid = 0;            // primitives with a finite, non-empty box
     bool parts = false;              // built over parts (ref_data, ref_geom) or spheres

@@ -231,7 +231,7 @@ __device__ __forceinline__ PartShape part_shape(const SceneDev& sc, uint32_t s, 
         return p;
     }
     const float q2 = b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
-    p.regular = g.bounded != 0u && fabsf(q2 - 1.0f) < 1e-3f;
+    p.regular = g.bounded != 0u && fabsf(q2 - 1.0f) < UNIT_SLACK;
     float r = g.bound_radius;
     if (type == FR_GEOM_MESH)
         r = r * fmaxf(q2, 1.0f) * 1.0001f;
@@ -528,6 +528,12 @@ constexpr uint64_t LIST_MIN_RAYS = 3u << 20;
 // cells (313k spheres at 186x97 with a lens, beams of several radii: 0.39 ms without lists, 1.79 ms
 // with them; no frame of 150 drawn ones with beams below this was slower by more than 1%).
 constexpr double LIST_WIDEST = 0.6;
+// Share of the references (1 in so many) that may be odd: nothing is known of how near one can be
+// hit, so every ray of the beam tests it, and a list of 15 of them is complete nowhere.  Preview of
+// 5000 primitives at 1000x700, cubes with quaternions of norm 0.95 among cubes: 8% of them 6.8 ms
+// with lists and 8.0 without, 30% 7.8 and 7.8, all 11.7 and 7.3; 20000 of a third that density, 8%
+// 8.1 and 8.4, 15% 8.4 and 8.3, 30% 9.0 and 8.2.
+constexpr uint32_t LIST_ODD_SHARE = 8;
 
 bool lists_possible(const FrameParams& P)
 {
@@ -541,6 +547,8 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
     const GridDev& G = P.scene.grid;
     if (G.nx <= 1 || G.ny <= 1 || G.nz <= 1)
         return false;  // a camera ray crosses only a cell or two of a flat layer
+    if (uint64_t(G.n_odd) * LIST_ODD_SHARE > G.n_refs)
+        return false;
     // the beam's radius in the middle of the grid: one pixel, and the lens away from the focus
     const CamK& k = P.cam;
     double rho = std::fabs(double(k.focal_h)) / k.height;
