@@ -854,6 +854,12 @@ fr_status prepare_grid(fr_scene* sc, fr_tracer* tr, int kind, uint32_t gi,
         sc->grid_key.clear();
         return cuda_fail(e, "building a sphere grid");
     }
+    uint64_t of_type[3] = {0, 0, 0};
+    for (const fr_geometry* g : parts)
+        of_type[g->type == FR_GEOM_SPHERE       ? 0
+                : g->type == FR_GEOM_POLYHEDRON ? 1
+                                                : 2] += g->n;
+    sc->grid.list_widest = list_widest(of_type[0], of_type[1], of_type[2]);
     sc->grid_key = key;
     sc->grid_geom = gi;
     sc->use_grid = sc->grid_report.built;
@@ -1064,6 +1070,7 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
         d.ihz = 1.0f / G.cell[2];
         d.geom = sc->grid_geom;
         d.n_valid = G.n_valid;
+        d.list_widest = G.list_widest;
         d.n_refs = G.n_refs;
         d.n_odd = G.n_odd;
         d.mean_radius = G.mean_radius;

@@ -86,6 +86,7 @@ struct GridDev {
     float ihx, ihy, ihz;  // 1 / cell size
     uint32_t geom;        // scene index of the sphere geometry
     uint32_t n_valid;     // primitives with a finite, non-empty box
+    float list_widest;    // see list_widest (render.hpp)
     uint32_t n_refs;
     uint32_t n_odd;       // references whose surface may lie outside their bounds (part_odd)
     float mean_radius;    // root of their mean cross-section / pi

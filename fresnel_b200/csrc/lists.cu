@@ -528,6 +528,19 @@ constexpr uint64_t LIST_MIN_RAYS = 3u << 20;
 // cells (313k spheres at 186x97 with a lens, beams of several radii: 0.39 ms without lists, 1.79 ms
 // with them; no frame of 150 drawn ones with beams below this was slower by more than 1%).
 constexpr double LIST_WIDEST = 0.6;
+// The same for scenes of polyhedra, and of cylinders, meshes and polygons alone: their bounds are
+// loose, so a list of 15 holds fewer that a ray meets, and no sphere's solid inside ends it.
+// Mixed scenes take the harmonic mean over their primitives, and few rays, over which the lists'
+// own time counts for more, the fourth root of their number less.  Against no lists, at 16M rays'
+// worth: Preview at 1000x700 (45M) of cubes at beams of 0.037 1.27x, 0.087 1.10x, 0.158 1.04x and
+// 0.177 0.78x; of cylinders 0.063 1.26x, 0.15 1.02x, 0.30 0.90x; of meshes 0.064 1.42x, 0.15 1.25x,
+// 0.31 0.97x; of spheres and bonds 0.20 1.33x; at 260x200 (3.3M) of cubes at 0.089 1.05x and 0.129
+// 0.73x, of cylinders 0.153 1.18x and 0.22 0.85x, of meshes 0.155 1.31x and 0.22 0.99x.  Path of
+// spheres and bonds at 640x480, 16 samples (4.9M), 0.18 1.09x and 0.29 0.94x, of the mixed scene
+// (five in seven are spheres) at 1280x720, 128 samples (118M), 0.35 1.15x.
+constexpr double LIST_WIDEST_POLYHEDRA = 0.1;
+constexpr double LIST_WIDEST_OTHERS = 0.2;
+constexpr double LIST_WIDEST_RAYS = 1 << 24;
 // Share of the references (1 in so many) that may be odd: nothing is known of how near one can be
 // hit, so every ray of the beam tests it, and a list of 15 of them is complete nowhere.  Preview of
 // 5000 primitives at 1000x700, cubes with quaternions of norm 0.95 among cubes: 8% of them 6.8 ms
@@ -562,7 +575,19 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
                             std::fabs(double(k.focal_d));
         rho = rho * s + 0.5 * std::fabs(double(k.aperture)) * std::max(std::fabs(1.0 - s), half);
     }
-    return rho <= LIST_WIDEST * G.mean_radius;
+    double widest = G.list_widest;
+    if (G.parts)
+        widest = std::min(LIST_WIDEST, widest * std::pow(double(P.w) * P.h * samples /
+                                                             LIST_WIDEST_RAYS, 0.25));
+    return rho <= widest * G.mean_radius;
+}
+
+float list_widest(uint64_t spheres, uint64_t polyhedra, uint64_t others)
+{
+    const double n = double(spheres + polyhedra + others);
+    return float(n > 0.0 ? n / (spheres / LIST_WIDEST + polyhedra / LIST_WIDEST_POLYHEDRA +
+                                others / LIST_WIDEST_OTHERS)
+                         : LIST_WIDEST);
 }
 
 void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStream_t st)

@@ -133,7 +133,10 @@ void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStrea
 // Per-pixel primitive lists of the frame's camera rays (beam.cuh: LIST_WORDS uint2 per pixel,
 // row by row), for scenes where lists are possible; lists_pay: `samples` camera rays per pixel are
 // expected to gain more than the lists cost.
+// list_widest: the beam radius, in mean primitive radii, up to which lists of a scene of so many
+// primitives of each type pay.
 bool lists_possible(const FrameParams& P);
+float list_widest(uint64_t spheres, uint64_t polyhedra, uint64_t others);
 bool lists_pay(const FrameParams& P, uint32_t samples);
 void launch_pixel_lists(const FrameParams& P, uint2* lists, cudaStream_t st);
 size_t pixel_list_words(const FrameParams& P);

@@ -65,3 +65,39 @@ def test_frames_with_lists(gpu_device, name):
         option("pixel_lists", 2)
     numpy.testing.assert_array_equal(got[0][0], got[1][0])
     assert (got[1][1] < 0.8 * got[0][1]) if used else (got[1][1] == got[0][1])
+
+
+def _spheres_and_bonds(dev, m=14):
+    rng = numpy.random.default_rng(4)
+    ijk = numpy.stack(numpy.meshgrid(*[numpy.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = ((ijk - (m - 1) / 2) * 2.0 + rng.uniform(-0.3, 0.3, (m**3, 3))).astype(numpy.float32)
+    scene = fresnel.Scene(dev, lights=fresnel.light.rembrandt())
+    fresnel.geometry.Sphere(scene, position=pos, radius=0.4, color=(0.4, 0.5, 0.6))
+    i = numpy.flatnonzero(ijk[:, 2] < m - 1)
+    fresnel.geometry.Cylinder(scene, points=numpy.stack([pos[i], pos[i + 1]], 1), radius=0.1,
+                              color=(0.3, 0.3, 0.8))
+    scene.camera = fresnel.camera.Orthographic(position=(4 * m, 4 * m, 4 * m), look_at=(0, 0, 0),
+                                               up=(0, 1, 0), height=3.6 * m)
+    return scene
+
+
+@pytest.mark.parametrize("kind,size,used", [
+    ("cubes", (1000, 700), True), ("cubes", (260, 200), False), ("cubes_dense", (260, 200), False),
+    ("bonds", (640, 480), True), ("bonds", (260, 200), False)])
+def test_beams_that_suit_the_primitives(gpu_device, kind, size, used):
+    """Lists over parts ask for thinner beams (more pixels) than lists over spheres, the thinner the
+    fewer rays there are."""
+    scene = (_spheres_and_bonds(gpu_device) if kind == "bonds" else
+             _cubes(gpu_device, n=500 if kind == "cubes" else 20000))
+    option = gpu_device._device.setOption
+    got = []
+    try:
+        for lists in (0, 2):
+            option("pixel_lists", lists)
+            t = fresnel.tracer.Preview(gpu_device, *size, anti_alias=True)
+            t.render(scene)
+            got.append((t.linear_output[:].copy(), t._tracer.getStats()["box_tests"]))
+    finally:
+        option("pixel_lists", 2)
+    numpy.testing.assert_array_equal(got[0][0], got[1][0])
+    assert (got[1][1] < 0.8 * got[0][1]) if used else (got[1][1] == got[0][1])
