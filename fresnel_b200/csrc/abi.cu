@@ -1133,6 +1133,7 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
     P.packet = sc->use_grid ? 0 : sc->dev->packet;
     P.refill = sc->dev->refill;
     P.preview_warp = sc->dev->preview_warp;
+    P.preview_rounds = P.scene.grid.n_cells == 0 || flat_layer(P.scene.grid);
     tr->last_grid = sc->use_grid ? (sc->grid.parts ? 2u : 1u) : 0u;
     const fr_user_camera& c = p->camera;
     float f_stop = preview ? std::numeric_limits<float>::infinity() : c.f_stop;  // no depth of field in preview
@@ -1164,11 +1165,9 @@ FrameParams frame_params(fr_tracer* tr, fr_scene* sc, const fr_render_params* p,
     return P;
 }
 
-// A grid one cell thick: its extension rays leave it at once, and the separate passes have nothing
-// to gain (10k polygons 800x800, 32 samples: 2.44 ms fused, 2.60 ms over packed queues).
-bool flat_layer(const GridDev& G) { return G.nx <= 1 || G.ny <= 1 || G.nz <= 1; }
-
-// Path slots from which extension rays go over packed queues (below, the launches cost more than
+// Path slots from which extension rays go over packed queues (but not those of a flat layer, where
+// separate passes have nothing to gain: 10k polygons 800x800, 32 samples: 2.44 ms fused, 2.60 ms
+// over packed queues; below, the launches cost more than
 // the fused bounce and tail kernels lose: frames of 2M slots and few hits 0.90-0.96x), and the
 // queue length below which the tail kernel follows the remaining paths (200k spheres 1024x768, 16
 // samples: 3.14 ms at 16k, 2.96 at 256k, 2.65 at 1.5M; 1M spheres 1080p: 46.3, 45.2, 44.6 ms).

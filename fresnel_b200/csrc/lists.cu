@@ -558,7 +558,7 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
     if (samples < LIST_MIN_SAMPLES || uint64_t(P.w) * P.h * samples < LIST_MIN_RAYS)
         return false;
     const GridDev& G = P.scene.grid;
-    if (G.nx <= 1 || G.ny <= 1 || G.nz <= 1)
+    if (flat_layer(G))
         return false;  // a camera ray crosses only a cell or two of a flat layer
     if (uint64_t(G.n_odd) * LIST_ODD_SHARE > G.n_refs)
         return false;

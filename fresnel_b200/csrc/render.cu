@@ -814,11 +814,13 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
         float avg = 0.0f;  // lanes 0-3 of the group: red, green, blue, alpha
         for (uint32_t base = 0; base < ns; base += G) {
             const uint32_t sample = base + gl;
-            // the warps of a block start each round together (every group of any block but the
-            // last has a pixel): the kernel is bound by instruction fetch (6 of 17 stall cycles on
-            // the cubes scene), which warps at the same place share (cubes Preview 4.94 -> 4.70 ms;
-            // groups taking pixel after pixel in a persistent grid instead, 6.3 ms)
-            if (base && blockIdx.x + 1u < gridDim.x)
+            // The warps of a block start each round together where their walks last alike: with
+            // lists, over trees and in flat layers (every group of any block but the last has a
+            // pixel).  The kernel is bound by instruction fetch (6 of 17 stall cycles on the cubes
+            // scene), which warps at the same place share: cubes Preview 4.94 -> 4.70 ms, 5k
+            // spheres in droplets 260x200 0.518 -> 0.501, 160k polygons 480x360 2.02 -> 1.89;
+            // groups taking pixel after pixel in a persistent grid instead, 6.3 ms.
+            if ((LISTS || P.preview_rounds) && base && blockIdx.x + 1u < gridDim.x)
                 __syncthreads();
             V3 o, d;
             Hit h;
@@ -859,7 +861,14 @@ __global__ void __launch_bounds__(256) k_preview_warp(FrameParams P, uint32_t aa
         if (gl == 0u)
             write_pixel(P, p, r, gr, b, al);
     }
-    flush_block(tc, P.tests);
+    // Without lists, walks of one warp may last several times those of another, and one that waits
+    // for the block's others holds registers the next block could start with: no barrier there,
+    // not even for the block's sums (60k aligned cylinders 500x400: 6.86 ms with both barriers,
+    // 6.75 without the rounds', 6.09 without either).
+    if constexpr (LISTS)
+        flush_block(tc, P.tests);
+    else
+        flush_counts(tc, P.tests);
     count_preview(P, ns);
 }
 

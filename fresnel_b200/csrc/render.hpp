@@ -28,6 +28,7 @@ struct FrameParams {
     int shade_blocks;        // 0: shade kernel as compiled; 3 or 4: register-limited variants
     int packet;              // 1: primary rays traced warp-cooperatively (4-wide trees)
     int refill;              // 1: extension rays with per-lane refill where refill_geom != -1
+    int preview_rounds;      // that kernel's warps start each round of samples together
     int preview_warp;        // 1: Preview with 32k samples per pixel traces one pixel per warp
     int refill_geom;         // -2: the scene's combined tree; >= 0: its one enabled geometry;
                              // -1: several per-geometry trees (refill not available)
@@ -161,6 +162,8 @@ void launch_traversal_compare(const SceneDev& sc, const float* rays, uint32_t n,
 constexpr uint32_t HIST_BINS = 512;
 void launch_histogram(const float4* linear, uint32_t n, uint32_t* counts, int num_sms,
                       cudaStream_t st);
+// A grid one cell thick: rays leave it at once.
+inline bool flat_layer(const GridDev& G) { return G.nx <= 1 || G.ny <= 1 || G.nz <= 1; }
 // Whether Preview traces a pixel's samples with a group of lanes.
 bool preview_groups(const FrameParams& P, uint32_t aa_n);
 // TracerDirect::render
