@@ -22,8 +22,8 @@
 
 namespace fr {
 
-// A pixel's list: LIST_WORDS uint2; word 0 is (entries, bits of the complete distance), the
-// others (slot, bits of the nearest distance a ray can be hit at).  Slots number the grid's
+// A pixel's list: LIST_WORDS uint2; word 0 is (entries, bits of the distance up to which the list
+// answers: it is complete, or every ray hit, nearer than that), the others (slot, bits of the nearest distance a ray can be hit at).  Slots number the grid's
 // references.  128 bytes: one line per pixel.
 constexpr uint32_t LIST_WORDS = 16;
 constexpr uint32_t LIST_MAX = LIST_WORDS - 1;

@@ -129,11 +129,12 @@ struct ListBuilder {
     }
     __device__ __forceinline__ void store(uint2* out) const
     {
-        // entries at or beyond `certain` or `complete` are never needed
+        // entries beyond `certain` or `complete` are never needed, and a ray that no entry answers
+        // nearer than that walks: only a list with neither bound can tell that a ray misses
         uint32_t m = n;
         while (m > 0u && __uint_as_float(e[(m - 1u) * 32u].y) > reach())
             --m;
-        out[0] = make_uint2(m, __float_as_uint(complete));
+        out[0] = make_uint2(m, __float_as_uint(reach()));
         for (uint32_t k = 0; k < m; ++k)
             out[k + 1u] = e[k * 32u];
     }
@@ -145,7 +146,8 @@ struct ListBuilder {
 struct SphereBounds {
     float reach;    // some ray may be accepted by the float test if the distance is at most
     float t_lo;     // this, and then not nearer than t_lo
-    float inner2;   // every ray is hit before t_hi if the squared distance is at most this
+    float inner2;   // every ray is hit before t_hi if the squared distance is at most this and
+                    // the centre lies ahead of the beam's origin
     float t_hi;
     float hi;       // no ray is hit beyond this
 };
@@ -174,11 +176,11 @@ __device__ __forceinline__ SphereBounds sphere_bounds(const Beam& b, bool parall
     return s;
 }
 
-// Squared distance of c from the beam's axis.
-__device__ __forceinline__ float axis_dist2(const Beam& b, V3 c)
+// Squared distance of c from the line of the beam's axis; tau: of its foot along the axis.
+__device__ __forceinline__ float axis_dist2(const Beam& b, V3 c, float& tau)
 {
     const V3 v = c - b.o;
-    const float tau = fmaf(v.x, b.d.x, fmaf(v.y, b.d.y, v.z * b.d.z));
+    tau = fmaf(v.x, b.d.x, fmaf(v.y, b.d.y, v.z * b.d.z));
     const float x = fmaf(-tau, b.d.x, v.x), y = fmaf(-tau, b.d.y, v.y), z = fmaf(-tau, b.d.z, v.z);
     return fmaf(x, x, fmaf(y, y, z * z));
 }
@@ -414,7 +416,8 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
                                 const SphereBounds sb =
                                     sphere_bounds(tb, parallel, spread, c, rad, pixel_radius);
                                 const float w = sb.reach + tb.over(sb.t_lo * (1.0f - 1.2f * tb.g), sb.hi);
-                                pass = axis_dist2(tb, c) <= w * w;
+                                float tau;
+                                pass = axis_dist2(tb, c, tau) <= w * w;
                                 rec = make_float4(c.x, c.y, c.z, sb.reach * sb.reach);
                                 bnd = make_float4(sb.t_lo, sb.inner2, sb.t_hi, 0.0f);
                             } else {
@@ -450,9 +453,10 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
                             float t_lo = u.x;
                             bool hit;
                             if (!PARTS || u.y != BOX) {
-                                const float a2 = axis_dist2(pb, c);
+                                float tau;
+                                const float a2 = axis_dist2(pb, c, tau);
                                 hit = a2 <= q.w;
-                                if (a2 <= u.y)
+                                if (a2 <= u.y && tau > 0.0f)
                                     L.certain = fminf(L.certain, u.z);
                             } else {
                                 const bool odd = q.w < 0.0f;

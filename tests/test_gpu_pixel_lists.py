@@ -115,3 +115,35 @@ def test_lists_give_the_walks_images(gpu_device, name, size):
         assert images[0][2][key] == images[1][2][key]
     if name == "grid" and size == (97, 61):  # the lists are in use
         assert images[1][2]["box_tests"] < 0.8 * images[0][2]["box_tests"]
+
+
+@pytest.mark.parametrize("bonds", [False, True])
+@pytest.mark.parametrize("half", [0.5, 2.0, 8.0])
+def test_lists_with_primitives_behind_the_camera(gpu_device, bonds, half):
+    """A camera among the spheres, from a moderate to a very wide angle: the line of a pixel's axis
+    also meets spheres behind the camera, which hide nothing."""
+    import fresnel_b200 as fresnel
+    rng = numpy.random.default_rng(12)
+    option = gpu_device._device.setOption
+    scene = fresnel.Scene(gpu_device, lights=fresnel.light.cloudy())
+    pos = rng.uniform(-6, 6, (400, 3)).astype(numpy.float32)
+    # one right behind the camera, in the cells around it, and none that holds it
+    pos = numpy.concatenate([pos[numpy.linalg.norm(pos, axis=1) > 1.2],
+                             [[-0.75, 0.02, 0.01]]]).astype(numpy.float32)
+    fresnel.geometry.Sphere(scene, position=pos, radius=0.5)
+    if bonds:
+        fresnel.geometry.Cylinder(scene, points=numpy.stack([pos[:60] * 1.3, pos[60:120]], 1),
+                                  radius=0.1)
+    scene.camera = fresnel.camera.Perspective(position=(0, 0, 0), look_at=(1, 0, 0), up=(0, 0, 1),
+                                              focal_length=1.0, height=2 * half)
+    images = []
+    try:
+        for lists in (0, 1):
+            option("pixel_lists", lists)
+            t = fresnel.tracer.Preview(gpu_device, 480, 320, anti_alias=True)
+            t.render(scene)
+            images.append((t.linear_output[:].copy(), t._tracer.getStats()["box_tests"]))
+    finally:
+        option("pixel_lists", 2)
+    numpy.testing.assert_array_equal(images[0][0], images[1][0])
+    assert images[1][1] < images[0][1]  # lists were in use
