@@ -12,7 +12,9 @@
 //     listed (the beam is widened by the jitter, the lens, and the rounding of the float tests);
 //   * the closest listed hit lies nearer than `complete` and its point lies inside the primitive's
 //     own bounding box by more than the walk's rounding, so that the walk, which tests every
-//     primitive whose box the ray enters before its closest hit, tests this one too.
+//     primitive whose box the ray enters before its closest hit, tests this one too; nor does a
+//     primitive that the walk may or may not test, depending on its order (parts_cell_test), lie
+//     closer.
 // Any other ray takes the walk itself (list_hit returns false), so images are identical with and
 // without lists.
 #ifndef FR_BEAM_CUH
@@ -118,8 +120,8 @@ __device__ __forceinline__ bool list_hit(const FrameParams& P, const uint2* list
             const uint2 c = __ldg(list + e);
             if (tmax < __uint_as_float(c.y))
                 break;
-            parts_cell_test<MASK & MASK_ALL>(sc, ray, c.x, c.x + 1u, tnear, tmax, hg, hp, last_g,
-                                             last_p, tc);
+            parts_cell_test<MASK & MASK_ALL, true>(sc, ray, c.x, c.x + 1u, tnear, tmax, hg, hp,
+                                                   last_g, last_p, tc);
         }
         if (hg == MISS)
             return complete == __int_as_float(0x7f800000);

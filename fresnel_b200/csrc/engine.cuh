@@ -828,6 +828,11 @@ __device__ __forceinline__ bool mixed_prim_t(const SceneDev& sc, const GeomDev& 
     return false;
 }
 
+// Distances that the test of a primitive of a grid over parts may be off by, per distance: a
+// cylinder's discriminant is off by up to 1.25e-6 of the squared distance, its root by 1.1e-3 of the
+// distance; doubled.
+constexpr float PART_SLACK = 2.2e-3f;
+
 // Leaf of a combined tree: each slot names its geometry; the primitive test is that geometry
 // type's (only the types in MASK are compiled in).
 template <uint32_t MASK>
@@ -872,7 +877,13 @@ __device__ __forceinline__ void leaf_test_mixed(const SceneDev& sc, const RayK& 
 // No primitive or instance is tested again right after itself (last_geom, last_prim: one
 // spanning several cells along the ray; its test and the acceptance are exact, so a repeat
 // could not change the hit).
-template <uint32_t MASK>
+//
+// A test's own distance may lie a little before the entry into the box (a grazed cylinder's is off by
+// up to 1.1e-3 of the distance, see PART_SLACK), so that whether a closer hit already known keeps
+// the primitive from being tested depends on the order of the tests.  LISTED: the references come in
+// another order than the walk's, and those whose boxes the segment ends just before are tested too;
+// the caller (list_hit) takes the walk where one of them is then the closest hit.
+template <uint32_t MASK, bool LISTED = false>
 __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& ray,
                                                 uint32_t first, uint32_t last, float tnear,
                                                 float& tmax, uint32_t& hit_geom,
@@ -880,6 +891,17 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
                                                 uint32_t& last_prim, TraceCount& tc)
 {
     tc.prim += last - first;
+    // distance up to which a box (corners lo, hi) is entered
+    const auto end = [&](V3 lo, V3 hi) {
+        if constexpr (LISTED) {
+            const V3 a = lo - ray.o, b = hi - ray.o;
+            return tmax + PART_SLACK * fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(b.x)),
+                                                   fmaxf(fabsf(a.y), fabsf(b.y))),
+                                             fmaxf(fabsf(a.z), fabsf(b.z)));
+        } else {
+            return tmax;
+        }
+    };
     for (uint32_t s = first; s < last; ++s) {
         // geometry index and type in one word (gather_parts): a sphere needs nothing from the
         // geometry table
@@ -904,7 +926,8 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
             if (!(dot(cr, cr) <= rp * rp * dd))
                 continue;  // the line misses the sphere
             const float reach = rp * sqrtf(dd);
-            if (bb + reach < 0.0f || bb - reach > tmax * dd)
+            if (bb + reach < 0.0f ||
+                bb - reach > end(pos - v3(rp, rp, rp), pos + v3(rp, rp, rp)) * dd)
                 continue;  // the sphere lies behind the origin or beyond the closest hit
             const uint32_t inst = __ldg(sc.order + s);
             if (gi == last_geom && inst == last_prim)
@@ -923,7 +946,7 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
                 lo = make_float4(lo.x - lpad, lo.y - lpad, lo.z - lpad, 0.0f);
                 hi = make_float4(hi.x + lpad, hi.y + lpad, hi.z + lpad, 0.0f);
                 float tentry;
-                if (!slab(lr, lo, hi, tmax, tentry))
+                if (!slab(lr, lo, hi, end(pos - v3(rp, rp, rp), pos + v3(rp, rp, rp)), tentry))
                     continue;
                 const V3 v0 = load3(g.vertices, 3 * f), v1 = load3(g.vertices, 3 * f + 1),
                          v2 = load3(g.vertices, 3 * f + 2);
@@ -964,7 +987,7 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
             lo = make_float4(lo.x - pad, lo.y - pad, lo.z - pad, 0.0f);
             hi = make_float4(hi.x + pad, hi.y + pad, hi.z + pad, 0.0f);
             float tentry;
-            if (!slab(ray, lo, hi, tmax, tentry))
+            if (!slab(ray, lo, hi, end(v3(lo.x, lo.y, lo.z), v3(hi.x, hi.y, hi.z)), tentry))
                 continue;
             const uint32_t prim = __ldg(sc.order + s);
             if (gi == last_geom && prim == last_prim)

@@ -196,7 +196,10 @@ __device__ __forceinline__ bool beam_box(const Beam& b, const RayK& axis, V3 c, 
     float t;
     if (!slab(axis, lo, hi, INF, t))
         return false;
-    t_lo = t * (1.0f - b.g) * (1.0f - 1e-5f);
+    // a test's own distance may lie before the box
+    const V3 v = c - b.o;
+    const float far = fmaxf(fmaxf(fabsf(v.x) + e.x, fabsf(v.y) + e.y), fabsf(v.z) + e.z) + R;
+    t_lo = fmaxf(t * (1.0f - b.g) * (1.0f - 1e-5f) - PART_SLACK * far, 0.0f);
     return true;
 }
 

@@ -208,11 +208,10 @@ struct PartsWalk : CellWalk {
         const V3 c = v3(q.x, q.y, q.z);
         radius = q.w;
         if (q.w < 0.0f) {
-            // widened by what the primitive's own test may be off by (see SPHERE_SLACK: a cylinder's
-            // discriminant is off by up to 1.25e-6 of the squared distance)
+            // widened by what the primitive's own test may be off by
             const V3 v = c - ray.o;
             const float far = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z));
-            radius = fmaf(far, 2.2e-3f, -q.w);
+            radius = fmaf(far, PART_SLACK, -q.w);
         }
         LineTest l(ray, c, radius);
         if (q.w < 0.0f) {

@@ -147,3 +147,32 @@ def test_lists_with_primitives_behind_the_camera(gpu_device, bonds, half):
         option("pixel_lists", 2)
     numpy.testing.assert_array_equal(images[0][0], images[1][0])
     assert images[1][1] < images[0][1]  # lists were in use
+
+
+@pytest.mark.parametrize("case", [(12, 2136, 0.2, 30.0), (7, 2046, 0.05, 0.0), (5, 5000, 0.05, 0.0)])
+def test_lists_of_grazed_cylinders(gpu_device, case):
+    """Long cylinders along an axis, seen obliquely from afar: the distance at which a ray that
+    grazes one meets it may lie just before its box, where another primitive is hit."""
+    import fresnel_b200 as fresnel
+    seed, n, radius, at = case
+    option = gpu_device._device.setOption
+    box = (n / 0.1) ** (1 / 3)
+    for k in range(6):
+        rng = numpy.random.default_rng([seed, k])
+        pos = rng.uniform(-box / 2, box / 2, (n, 3)) + at
+        axis = numpy.array([1.0, 0, 0]) + 1e-3 * rng.normal(size=(n, 3))
+        scene = fresnel.Scene(gpu_device, lights=fresnel.light.cloudy())
+        fresnel.geometry.Cylinder(scene, points=numpy.stack([pos, pos + 4 * axis], 1).astype(
+            numpy.float32), radius=(radius * rng.uniform(0.5, 1.5, n)).astype(numpy.float32))
+        scene.camera = fresnel.camera.Orthographic(
+            position=numpy.array([at] * 3) + 6 * box / math.sqrt(3), look_at=[at] * 3,
+            up=(0.1, 1, 0.05), height=1.2 * box)
+        hits = []
+        try:
+            for lists in (0, 1):
+                option("pixel_lists", lists)
+                t = fresnel.tracer.Preview(gpu_device, 320, 240, anti_alias=True)
+                hits.append(numpy.array(t._tracer.renderHitIds(scene._scene)))
+        finally:
+            option("pixel_lists", 2)
+        assert (hits[0] != hits[1]).any(-1).sum() == 0
