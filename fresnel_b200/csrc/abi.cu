@@ -854,12 +854,10 @@ fr_status prepare_grid(fr_scene* sc, fr_tracer* tr, int kind, uint32_t gi,
         sc->grid_key.clear();
         return cuda_fail(e, "building a sphere grid");
     }
-    uint64_t of_type[3] = {0, 0, 0};
+    uint64_t of_type[5] = {0, 0, 0, 0, 0};
     for (const fr_geometry* g : parts)
-        of_type[g->type == FR_GEOM_SPHERE       ? 0
-                : g->type == FR_GEOM_POLYHEDRON ? 1
-                                                : 2] += g->n;
-    sc->grid.list_widest = list_widest(of_type[0], of_type[1], of_type[2]);
+        of_type[g->type] += g->n;
+    sc->grid.list_widest = list_widest(of_type, sc->grid.free_cells);
     sc->grid_key = key;
     sc->grid_geom = gi;
     sc->use_grid = sc->grid_report.built;

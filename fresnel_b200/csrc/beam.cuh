@@ -12,9 +12,8 @@
 //     listed (the beam is widened by the jitter, the lens, and the rounding of the float tests);
 //   * the closest listed hit lies nearer than `complete` and its point lies inside the primitive's
 //     own bounding box by more than the walk's rounding, so that the walk, which tests every
-//     primitive whose box the ray enters before its closest hit, tests this one too; nor does a
-//     primitive that the walk may or may not test, depending on its order (parts_cell_test), lie
-//     closer.
+//     primitive whose box the ray enters before its closest hit, tests this one too; and the
+//     list holds every primitive that the walk may test before it ends (parts_cell_test).
 // Any other ray takes the walk itself (list_hit returns false), so images are identical with and
 // without lists.
 #ifndef FR_BEAM_CUH
@@ -25,8 +24,9 @@
 namespace fr {
 
 // A pixel's list: LIST_WORDS uint2; word 0 is (entries, bits of the distance up to which the list
-// answers: it is complete, or every ray hit, nearer than that), the others (slot, bits of the nearest distance a ray can be hit at).  Slots number the grid's
-// references.  128 bytes: one line per pixel.
+// answers: it is complete, or every ray hit, nearer than that), the others (slot, bits of the nearest
+// distance a ray can be hit at: over parts, of the cells of any but spheres).  Slots number the
+// grid's references.  128 bytes: one line per pixel.
 constexpr uint32_t LIST_WORDS = 16;
 constexpr uint32_t LIST_MAX = LIST_WORDS - 1;
 

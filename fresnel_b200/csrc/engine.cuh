@@ -833,6 +833,22 @@ __device__ __forceinline__ bool mixed_prim_t(const SceneDev& sc, const GeomDev& 
 // distance; doubled.
 constexpr float PART_SLACK = 2.2e-3f;
 
+// The box lo, hi (padded beyond the rounding of the cells' planes) widened to the cells it lies in.
+__device__ __forceinline__ void cells_of(const GridDev& G, float4& lo, float4& hi)
+{
+    lo.x = fmaf(floorf((lo.x - G.lox) * G.ihx), G.hx, G.lox);
+    lo.y = fmaf(floorf((lo.y - G.loy) * G.ihy), G.hy, G.loy);
+    lo.z = fmaf(floorf((lo.z - G.loz) * G.ihz), G.hz, G.loz);
+    hi.x = fmaf(floorf((hi.x - G.lox) * G.ihx) + 1.0f, G.hx, G.lox);
+    hi.y = fmaf(floorf((hi.y - G.loy) * G.ihy) + 1.0f, G.hy, G.loy);
+    hi.z = fmaf(floorf((hi.z - G.loz) * G.ihz) + 1.0f, G.hz, G.loz);
+    const float pad = 2e-6f * fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)),
+                                          fmaxf(fabsf(lo.y), fabsf(hi.y))),
+                                    fmaxf(fabsf(lo.z), fabsf(hi.z)));
+    lo = make_float4(lo.x - pad, lo.y - pad, lo.z - pad, 0.0f);
+    hi = make_float4(hi.x + pad, hi.y + pad, hi.z + pad, 0.0f);
+}
+
 // Leaf of a combined tree: each slot names its geometry; the primitive test is that geometry
 // type's (only the types in MASK are compiled in).
 template <uint32_t MASK>
@@ -878,11 +894,13 @@ __device__ __forceinline__ void leaf_test_mixed(const SceneDev& sc, const RayK& 
 // spanning several cells along the ray; its test and the acceptance are exact, so a repeat
 // could not change the hit).
 //
-// A test's own distance may lie a little before the entry into the box (a grazed cylinder's is off by
-// up to 1.1e-3 of the distance, see PART_SLACK), so that whether a closer hit already known keeps
-// the primitive from being tested depends on the order of the tests.  LISTED: the references come in
-// another order than the walk's, and those whose boxes the segment ends just before are tested too;
-// the caller (list_hit) takes the walk where one of them is then the closest hit.
+// A test may accept a ray outside its primitive (a cylinder's discriminant is off by up to 1.25e-6 of
+// the squared distance; a polyhedron's stops where its entry and exit are equal, without the planes
+// left), and so at a distance before the entry into the box.  Whether a closer hit already known
+// keeps such a primitive from being tested then depends on the order of the tests.  LISTED: the
+// references come in another order than the walk's, and every primitive is tested that the walk
+// may test: one whose box the line meets at all and whose cells the segment (0, tmax) reaches.
+// Where the closest hit lies outside its box, the caller (list_hit) takes the walk.
 template <uint32_t MASK, bool LISTED = false>
 __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& ray,
                                                 uint32_t first, uint32_t last, float tnear,
@@ -891,16 +909,17 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
                                                 uint32_t& last_prim, TraceCount& tc)
 {
     tc.prim += last - first;
-    // distance up to which a box (corners lo, hi) is entered
-    const auto end = [&](V3 lo, V3 hi) {
-        if constexpr (LISTED) {
-            const V3 a = lo - ray.o, b = hi - ray.o;
-            return tmax + PART_SLACK * fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(b.x)),
-                                                   fmaxf(fabsf(a.y), fabsf(b.y))),
-                                             fmaxf(fabsf(a.z), fabsf(b.z)));
-        } else {
-            return tmax;
-        }
+    // whether the primitive with the box lo, hi is tested
+    const auto enters = [&](float4 lo, float4 hi) {
+        float te;
+        if constexpr (!LISTED)
+            return slab(ray, lo, hi, tmax, te);
+        if (!slab(ray, lo, hi, __int_as_float(0x7f800000), te))
+            return false;
+        if (te <= tmax)
+            return true;
+        cells_of(sc.grid, lo, hi);
+        return slab(ray, lo, hi, tmax, te);
     };
     for (uint32_t s = first; s < last; ++s) {
         // geometry index and type in one word (gather_parts): a sphere needs nothing from the
@@ -926,8 +945,9 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
             if (!(dot(cr, cr) <= rp * rp * dd))
                 continue;  // the line misses the sphere
             const float reach = rp * sqrtf(dd);
-            if (bb + reach < 0.0f ||
-                bb - reach > end(pos - v3(rp, rp, rp), pos + v3(rp, rp, rp)) * dd)
+            if (bb + reach < 0.0f || (!LISTED && bb - reach > tmax * dd) ||
+                (LISTED && !enters(make_float4(pos.x - rp, pos.y - rp, pos.z - rp, 0.0f),
+                                   make_float4(pos.x + rp, pos.y + rp, pos.z + rp, 0.0f))))
                 continue;  // the sphere lies behind the origin or beyond the closest hit
             const uint32_t inst = __ldg(sc.order + s);
             if (gi == last_geom && inst == last_prim)
@@ -946,7 +966,7 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
                 lo = make_float4(lo.x - lpad, lo.y - lpad, lo.z - lpad, 0.0f);
                 hi = make_float4(hi.x + lpad, hi.y + lpad, hi.z + lpad, 0.0f);
                 float tentry;
-                if (!slab(lr, lo, hi, end(pos - v3(rp, rp, rp), pos + v3(rp, rp, rp)), tentry))
+                if (!slab(lr, lo, hi, LISTED ? __int_as_float(0x7f800000) : tmax, tentry))
                     continue;
                 const V3 v0 = load3(g.vertices, 3 * f), v1 = load3(g.vertices, 3 * f + 1),
                          v2 = load3(g.vertices, 3 * f + 2);
@@ -986,8 +1006,7 @@ __device__ __forceinline__ void parts_cell_test(const SceneDev& sc, const RayK& 
             const float pad = 1e-4f * scale + 1e-5f;
             lo = make_float4(lo.x - pad, lo.y - pad, lo.z - pad, 0.0f);
             hi = make_float4(hi.x + pad, hi.y + pad, hi.z + pad, 0.0f);
-            float tentry;
-            if (!slab(ray, lo, hi, end(v3(lo.x, lo.y, lo.z), v3(hi.x, hi.y, hi.z)), tentry))
+            if (!enters(lo, hi))
                 continue;
             const uint32_t prim = __ldg(sc.order + s);
             if (gi == last_geom && prim == last_prim)

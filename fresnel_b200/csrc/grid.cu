@@ -465,6 +465,7 @@ cudaError_t build_cells(const Src& src, uint32_t n, const Reasons& why, const Gr
         return cudaSuccess;
     }
     out.mean_radius = float(std::sqrt(mean_r2));
+    out.free_cells = mean_r2 > 0.0 ? float(volume / (rep.n_valid * pi * mean_r2) / h_mean) : 0.0f;
     out.n_valid = rep.n_valid;
     for (int k = 0; k < 3; ++k) {
         out.dims[k] = dims[k];

@@ -26,6 +26,7 @@ struct GridBuffers {
     uint32_t n_odd = 0;              // of them, those whose surface may lie outside their bounds
     float mean_radius = 0.0f;        // root of the mean cross-section / pi of the primitives
     uint32_t n_valid = 0;            // primitives with a finite, non-empty box
+    float free_cells = 0.0f;         // cells along a ray between two primitives' boxes
     float list_widest = 0.0f;        // widest beam for pixel lists, in mean radii (render.hpp)
     bool parts = false;              // built over parts (ref_data, ref_geom) or spheres
     uint32_t dims[3] = {0, 0, 0};

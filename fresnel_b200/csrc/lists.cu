@@ -185,9 +185,10 @@ __device__ __forceinline__ float axis_dist2(const Beam& b, V3 c, float& tau)
     return fmaf(x, x, fmaf(y, y, z * z));
 }
 
-// The same for a box (centre c, half extents e): the axis against the box widened by R.
+// The same for a box (centre c, half extents e): the axis against the box widened by R; t_lo: some
+// ray may reach a cell that the box lies in from there on.
 __device__ __forceinline__ bool beam_box(const Beam& b, const RayK& axis, V3 c, V3 e, float R,
-                                         float& t_lo)
+                                         const GridDev& G, float& t_lo)
 {
     const float scale = fmaxf(fmaxf(fabsf(c.x) + e.x, fabsf(c.y) + e.y), fabsf(c.z) + e.z);
     const float w = R + 2e-4f * scale + 2e-5f;  // beyond the padding of the walk's own box test
@@ -196,10 +197,13 @@ __device__ __forceinline__ bool beam_box(const Beam& b, const RayK& axis, V3 c, 
     float t;
     if (!slab(axis, lo, hi, INF, t))
         return false;
-    // a test's own distance may lie before the box
-    const V3 v = c - b.o;
-    const float far = fmaxf(fmaxf(fabsf(v.x) + e.x, fabsf(v.y) + e.y), fabsf(v.z) + e.z) + R;
-    t_lo = fmaxf(t * (1.0f - b.g) * (1.0f - 1e-5f) - PART_SLACK * far, 0.0f);
+    const float p = w - R;  // the padding alone
+    float4 cl = make_float4(c.x - e.x - p, c.y - e.y - p, c.z - e.z - p, 0.0f);
+    float4 ch = make_float4(c.x + e.x + p, c.y + e.y + p, c.z + e.z + p, 0.0f);
+    cells_of(G, cl, ch);
+    slab(axis, make_float4(cl.x - w, cl.y - w, cl.z - w, 0.0f),
+         make_float4(ch.x + w, ch.y + w, ch.z + w, 0.0f), INF, t);
+    t_lo = t * (1.0f - b.g) * (1.0f - 1e-5f);
     return true;
 }
 
@@ -425,7 +429,7 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
                                 bnd = make_float4(sb.t_lo, sb.inner2, sb.t_hi, 0.0f);
                             } else {
                                 float t_lo;
-                                pass = beam_box(tb, tile_axis, c, sh.e, tile_R, t_lo);
+                                pass = beam_box(tb, tile_axis, c, sh.e, tile_R, G, t_lo);
                                 rec = make_float4(c.x, c.y, c.z, sh.e.x);
                                 bnd = make_float4(sh.e.y, BOX, sh.e.z, 0.0f);
                             }
@@ -463,7 +467,8 @@ __global__ void __launch_bounds__(128, 6) k_pixel_lists_grid(FrameParams P, uint
                                     L.certain = fminf(L.certain, u.z);
                             } else {
                                 const bool odd = q.w < 0.0f;
-                                hit = beam_box(pb, axis, c, v3(odd ? -q.w : q.w, u.x, u.z), R, t_lo);
+                                hit = beam_box(pb, axis, c, v3(odd ? -q.w : q.w, u.x, u.z), R, G,
+                                               t_lo);
                                 if (odd)
                                     t_lo = 0.0f;
                             }
@@ -535,18 +540,19 @@ constexpr uint64_t LIST_MIN_RAYS = 3u << 20;
 // cells (313k spheres at 186x97 with a lens, beams of several radii: 0.39 ms without lists, 1.79 ms
 // with them; no frame of 150 drawn ones with beams below this was slower by more than 1%).
 constexpr double LIST_WIDEST = 0.6;
-// The same for scenes of polyhedra, and of cylinders, meshes and polygons alone: their bounds are
-// loose, so a list of 15 holds fewer that a ray meets, and no sphere's solid inside ends it.
-// Mixed scenes take the harmonic mean over their primitives, and few rays, over which the lists'
-// own time counts for more, the fourth root of their number less.  Against no lists, at 16M rays'
-// worth: Preview at 1000x700 (45M) of cubes at beams of 0.037 1.27x, 0.087 1.10x, 0.158 1.04x and
-// 0.177 0.78x; of cylinders 0.063 1.26x, 0.15 1.02x, 0.30 0.90x; of meshes 0.064 1.42x, 0.15 1.25x,
-// 0.31 0.97x; of spheres and bonds 0.20 1.33x; at 260x200 (3.3M) of cubes at 0.089 1.05x and 0.129
-// 0.73x, of cylinders 0.153 1.18x and 0.22 0.85x, of meshes 0.155 1.31x and 0.22 0.99x.  Path of
-// spheres and bonds at 640x480, 16 samples (4.9M), 0.18 1.09x and 0.29 0.94x, of the mixed scene
-// (five in seven are spheres) at 1280x720, 128 samples (118M), 0.35 1.15x.
-constexpr double LIST_WIDEST_POLYHEDRA = 0.1;
-constexpr double LIST_WIDEST_OTHERS = 0.2;
+// The same for the other types, per cell that a ray crosses between two of their boxes: a list then
+// also holds what lies in the cells of what it meets (parts_cell_test), the more the closer
+// together the boxes are, no sphere's solid inside ends it, and a box holds less of a cylinder than
+// of a polyhedron or a mesh.  Scenes of several types take the harmonic mean over their primitives,
+// and few rays, over which the lists' own time counts for more, the fourth root of their number
+// less.  Preview at 1000x700 against no lists: 20k cubes at 0.3 per unit volume (0.57 cells), beams
+// of 0.087, 0.90x; 500 of them (0.025) 1.45x; 5k at 1.0 (0.25 cells, 0.037) 0.94x; a crystal at 0.24
+// (0.65 cells, 0.068) 1.23x.  Cylinders at 0.3 (1.7 cells) 0.044 1.76x and 0.15 0.89x; meshes 0.044
+// 1.41x and 0.15 1.05x, at 1.0 (0.77 cells) 0.064 1.17x.  Spheres and bonds (2.9 cells) 0.2 1.20x; the
+// mixed scene (five in seven are spheres, 1.8 cells) in a Path image of 118M rays, 0.35, 1.15x.
+constexpr double LIST_WIDEST_SOLIDS = 0.1;
+constexpr double LIST_WIDEST_CYLINDERS = 0.055;
+constexpr double LIST_WIDEST_PARTS = 0.12;  // (cubes at 0.05, 1.9 cells, 0.16: 0.93x)
 constexpr double LIST_WIDEST_RAYS = 1 << 24;
 // Share of the references (1 in so many) that may be odd: nothing is known of how near one can be
 // hit, so every ray of the beam tests it, and a list of 15 of them is complete nowhere.  Preview of
@@ -589,12 +595,21 @@ bool lists_pay(const FrameParams& P, uint32_t samples)
     return rho <= widest * G.mean_radius;
 }
 
-float list_widest(uint64_t spheres, uint64_t polyhedra, uint64_t others)
+float list_widest(const uint64_t (&of_type)[5], float free_cells)
 {
-    const double n = double(spheres + polyhedra + others);
-    return float(n > 0.0 ? n / (spheres / LIST_WIDEST + polyhedra / LIST_WIDEST_POLYHEDRA +
-                                others / LIST_WIDEST_OTHERS)
-                         : LIST_WIDEST);
+    double n = 0.0, inverse = 0.0;
+    for (int type = 0; type < 5; ++type) {
+        const bool solid = type == FR_GEOM_POLYHEDRON || type == FR_GEOM_MESH;
+        const double widest =
+            type == FR_GEOM_SPHERE
+                ? LIST_WIDEST
+                : std::min(LIST_WIDEST_PARTS, double(free_cells) * (solid ? LIST_WIDEST_SOLIDS
+                                                                          : LIST_WIDEST_CYLINDERS));
+        n += double(of_type[type]);
+        if (of_type[type])
+            inverse += of_type[type] / std::max(widest, 1e-6);
+    }
+    return float(n > 0.0 ? n / inverse : LIST_WIDEST);
 }
 
 void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStream_t st)

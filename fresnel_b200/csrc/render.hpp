@@ -135,9 +135,9 @@ void launch_part_bounds(const SceneDev& sc, uint32_t n, float4* bound, cudaStrea
 // row by row), for scenes where lists are possible; lists_pay: `samples` camera rays per pixel are
 // expected to gain more than the lists cost.
 // list_widest: the beam radius, in mean primitive radii, up to which lists of a scene of so many
-// primitives of each type pay.
+// primitives of each type (FR_GEOM_*) pay, given GridBuffers::free_cells.
 bool lists_possible(const FrameParams& P);
-float list_widest(uint64_t spheres, uint64_t polyhedra, uint64_t others);
+float list_widest(const uint64_t (&of_type)[5], float free_cells);
 bool lists_pay(const FrameParams& P, uint32_t samples);
 void launch_pixel_lists(const FrameParams& P, uint2* lists, cudaStream_t st);
 size_t pixel_list_words(const FrameParams& P);

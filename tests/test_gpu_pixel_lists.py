@@ -176,3 +176,42 @@ def test_lists_of_grazed_cylinders(gpu_device, case):
         finally:
             option("pixel_lists", 2)
         assert (hits[0] != hits[1]).any(-1).sum() == 0
+
+
+def test_lists_of_cylinders_among_polyhedra(gpu_device):
+    """Short cylinders among bricks, seen from afar: a ray accepted beside a cylinder can meet its box
+    only behind the next brick, so that whether the walk tests the cylinder depends on which of
+    the two it comes to first."""
+    import fresnel_b200 as fresnel
+    from fresnel_b200 import workloads
+    option = gpu_device._device.setOption
+    found = 0
+    for seed in range(3):
+        rng = numpy.random.default_rng([78, seed])
+        scene = fresnel.Scene(gpu_device, lights=fresnel.light.cloudy())
+        n, box = 4800, 30.0
+        info = workloads.unit_cube_planes()
+        info["face_origin"] = (info["face_origin"] * (0.2, 1, 1)).astype(numpy.float32)
+        info["radius"] = 0.71415
+        pos = rng.uniform(-box / 2, box / 2, (n, 3))
+        d = rng.normal(size=(n, 3))
+        d /= numpy.linalg.norm(d, axis=1, keepdims=True)
+        fresnel.geometry.Cylinder(scene, points=numpy.stack([pos, pos + d], 1).astype(numpy.float32),
+                                  radius=0.1)
+        fresnel.geometry.ConvexPolyhedron(
+            scene, info, position=rng.uniform(-box / 2, box / 2, (n, 3)).astype(numpy.float32),
+            orientation=workloads.random_quaternions(rng, n))
+        scene.camera = fresnel.camera.Perspective(position=(0, 0, 6 * box), look_at=(0, 0, 0),
+                                                  up=(0.1, 1, 0.07), focal_length=1.0,
+                                                  height=1 / 6)
+        hits = []
+        try:
+            for lists in (0, 1):
+                option("pixel_lists", lists)
+                t = fresnel.tracer.Preview(gpu_device, 640, 361, anti_alias=True)
+                t.seed = seed
+                hits.append(numpy.array(t._tracer.renderHitIds(scene._scene)))
+        finally:
+            option("pixel_lists", 2)
+        found += (hits[0] != hits[1]).any(-1).sum()
+    assert found == 0
