@@ -789,7 +789,9 @@ def main():
         # without shade launches each bounce traces and shades in one kernel
         primary_name = "k_path_primary_shade" if dd.getOption("fuse_shade") else "k_path_primary"
         ext_name = "k_path_bounce" if st["shade_launches"] == 0 else "k_path_extend"
-        if st.get("grid", 0) and st["shade_launches"] and dd.getOption("wave"):
+        if (st.get("grid", 0) and st["shade_launches"] and dd.getOption("wave")
+                and dd.getOption("fuse_shade") == 1 and dd.getOption("tail") >= 0
+                and not dd.getOption("refill")):
             # packed queues: a pass traces and one shades, then one tail launch does both
             ext_name = "k_wave_trace+k_wave_tail"
         if ext_name == "k_path_bounce" and dd.getOption("tail") >= 0:
