@@ -101,3 +101,60 @@ def test_beams_that_suit_the_primitives(gpu_device, kind, size, used):
         option("pixel_lists", 2)
     numpy.testing.assert_array_equal(got[0][0], got[1][0])
     assert (got[1][1] < 0.8 * got[0][1]) if used else (got[1][1] == got[0][1])
+
+
+def test_trees_take_no_lists(gpu_device):
+    """Lists are of grid references: over trees the option changes nothing."""
+    scene = _cubes(gpu_device)
+    option = gpu_device._device.setOption
+    option("accel", 0)
+    counts = []
+    try:
+        for lists in (0, 1):
+            option("pixel_lists", lists)
+            t = fresnel.tracer.Preview(gpu_device, 160, 120, anti_alias=True)
+            t.render(scene)
+            counts.append(t._tracer.getStats()["box_tests"])
+    finally:
+        option("pixel_lists", 2)
+        option("accel", 2)
+    assert counts[0] == counts[1] > 0
+
+
+def test_path_images_over_parts_take_lists(gpu_device):
+    scene = _spheres_and_bonds(gpu_device)  # (beams of 0.13 mean radii, 21M rays: 0.2 allowed)
+    option = gpu_device._device.setOption
+    counts = []
+    try:
+        for lists in (0, 2):
+            option("pixel_lists", lists)
+            t = fresnel.tracer.Path(gpu_device, 1000, 700)
+            t.seed = 3
+            t.sample(scene, 30)
+            counts.append((t._tracer.getStats()["box_tests"], t.linear_output[:].copy()))
+    finally:
+        option("pixel_lists", 2)
+    assert counts[1][0] < counts[0][0]
+    numpy.testing.assert_array_equal(counts[0][1], counts[1][1])
+
+
+def test_tiles_that_reach_the_budget(gpu_device):
+    """A very wide tile over many small spheres ends after a few thousand references; its lists then
+    answer up to there only."""
+    rng = numpy.random.default_rng(6)
+    scene = fresnel.Scene(gpu_device, lights=fresnel.light.cloudy())
+    fresnel.geometry.Sphere(scene, position=rng.uniform(-20, 20, (60000, 3)).astype(numpy.float32),
+                            radius=0.15)
+    scene.camera = fresnel.camera.Orthographic(position=(50, 60, 70), look_at=(0, 0, 0),
+                                               up=(0, 1, 0), height=70.0)
+    option = gpu_device._device.setOption
+    images = []
+    try:
+        for lists in (0, 1):
+            option("pixel_lists", lists)
+            t = fresnel.tracer.Preview(gpu_device, 40, 24, anti_alias=True)
+            t.render(scene)
+            images.append(t.linear_output[:].copy())
+    finally:
+        option("pixel_lists", 2)
+    numpy.testing.assert_array_equal(images[0], images[1])

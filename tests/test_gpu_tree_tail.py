@@ -51,3 +51,30 @@ def test_tail_gives_the_passes_images(gpu_device, name):
     finally:
         option("tail", 1)
         option("accel", 2)
+
+
+def test_tail_kernel_runs(gpu_device):
+    """The cases above compare two routes only if the tail takes the place of later passes."""
+    import fresnel_b200 as fresnel
+    n, size, samples, at = CASES["cluster"]
+    option = gpu_device._device.setOption
+    rng = numpy.random.default_rng(21)
+    option("accel", 0)
+    launches = {}
+    try:
+        scene = fresnel.Scene(gpu_device, lights=fresnel.light.cloudy())
+        fresnel.geometry.Sphere(scene, position=rng.normal(0, 3, (n, 3)).astype(numpy.float32),
+                                radius=0.5)
+        scene.camera = fresnel.camera.Perspective(position=(0, 0, at), look_at=(0, 0, 0),
+                                                  up=(0, 1, 0), focal_length=0.5, height=0.5)
+        for tail in (-1, 0, 1, 3):
+            option("tail", tail)
+            t = fresnel.tracer.Path(gpu_device, *size)
+            t.sample(scene, samples)
+            launches[tail] = t._tracer.getStats()["kernel_launches"]
+    finally:
+        option("tail", 1)
+        option("accel", 2)
+    # camera pass, tail, fold, and two launches for each pass before the tail
+    assert launches[0] == 3 and launches[1] == 5 and launches[3] == 9
+    assert launches[-1] > launches[3]
