@@ -16,8 +16,9 @@
 // Against the fused bounce and tail kernels: 1M spheres 1080p, 256 samples 54.4 -> 44.4 ms a frame;
 // 1000 spheres with 32 light samples 50.8 -> 34.5 ms; 200k spheres, 16 samples 2.87 -> 2.72 ms.
 // The mixed scene of 280k primitives, 1280x720, 128 samples: 51.4 -> 31.3 ms.
-// What bounds k_wave_trace now: issue (72%), with 15 of 32 lanes active on average (a lane's
-// iteration takes the test, the square root or the step, and not all need each).
+// What bounds k_wave_trace now: issue (62-72%), with 13 to 15 of 32 lanes active on average (a lane's
+// iteration takes the test, the square root or the step, and not all need each); over parts 7 to 8
+// lanes at 66%.
 #include "path_device.cuh"
 
 namespace fr {

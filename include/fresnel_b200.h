@@ -208,7 +208,8 @@ FR_API fr_status fr_device_timer_stop(fr_device* dev, float* ms);
  *                   them: 0: never (every ray walks the acceleration structure); 1: for every
  *                   scene traced through a grid; 2 (default): where they are expected to pay
  *                   (at least 16 samples per pixel, 3 million camera rays, beams thinner than
- *                   the primitives).  The same images in every case.  The lists take 128
+ *                   the primitives: over parts the thinner the less room a box leaves and the
+ *                   fewer rays there are).  The same images in every case.  The lists take 128
  *                   bytes per pixel of the largest image so far (265 MB at 1920x1080), in a
  *                   batch of each of up to 32 renders that run side by side; they,
  *                   and the second record queue of "wave", are kept between renders and given
@@ -386,9 +387,10 @@ typedef struct fr_batch_stats {
     uint32_t waves;               /* wavefronts (renders that fit the path state together) */
     uint64_t graph_launches;
     uint64_t graph_captures;
-    uint64_t kernel_launches;     /* kernels executed, inside the graphs or beside them (renders
-                                     of half a million path slots and more run on streams of
-                                     their own instead of in the graph) */
+    uint64_t kernel_launches;     /* kernels executed, inside the graphs or beside them (batches
+                                     over grids that are not flat run on streams instead of in
+                                     the graph from 512k path slots a render on average, 2M
+                                     and 196k expected hits with several light samples) */
     uint64_t shade_extend_pairs;  /* device-side loop passes (two bounces each) */
     uint64_t box_tests, prim_tests;
     float last_ms;                /* device time of the last fr_batch_render */
