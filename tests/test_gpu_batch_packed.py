@@ -108,8 +108,10 @@ def test_batches_that_miss_take_the_graph(gpu_device, lights, height, packed):
 def test_packed_batch_lists_take_a_lane_each(gpu_device):
     """The pixel lists of a batch's renders take memory for those that run at once (32 streams), not
     for all of its renders."""
+    import gc
     import torch
     import fresnel_b200 as fresnel
+    gc.collect()  # (what earlier tests left would be freed between the two readings)
     dev = fresnel.Device(mode="gpu")
     scene = _scenes(dev)[0]
     batch = fresnel.tracer.PathBatch(dev)
